@@ -474,20 +474,6 @@ def _op_sort_large(ctx, peak, reps):
     f = R.gen_uniform_rows(n, [32, 64], PL.C2_SEED + 2, [0, 100], [PL.C2_D2_ROWS, 10_000_000], device=ctx.dev)
     out = {"sort_tuples_%s_16B_on_fk" % tag: _sort_line(f, 16, 64, 96, 3, peak, flags=R.SORT_SKIP_TRIVIAL, passes=3,
                                                         note="fk < 2^24: the top digit is constant and skipped")}
-    R.tune_force(R.TUNE_SORT_PASS, 1)
-    try:
-        out["sort_tuples_%s_16B_on_fk_onesweep_pass" % tag] = _sort_line(f, 16, 64, 96, 3, peak,
-                                                                         flags=R.SORT_SKIP_TRIVIAL, passes=3,
-                                                                         note="the pipelined onesweep pass")
-    finally:
-        R.tune_force(R.TUNE_SORT_PASS, -1)
-    R.tune_force(R.TUNE_SORT_PASS, 4)
-    try:
-        out["sort_tuples_%s_16B_on_fk_match_rank" % tag] = _sort_line(f, 16, 64, 96, 3, peak,
-                                                                      flags=R.SORT_SKIP_TRIVIAL, passes=3,
-                                                                      note="per-tile pass ranking with match_any")
-    finally:
-        R.tune_force(R.TUNE_SORT_PASS, -1)
     del f
     keys = R.gen_uniform_rows(n, [32], 0x5EED0101, [0], [1 << 32], device=ctx.dev)
     out["sort_keys_%s_u32" % tag] = _sort_line(keys.view(torch.uint8).view(n, 4), 4, 0, 32, 3, peak,

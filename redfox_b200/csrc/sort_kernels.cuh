@@ -1,8 +1,7 @@
 // sort_kernels.cuh -- stable LSD radix sort of packed keys (with optional values):
-// one histogram pass over the keys for every digit, then one "onesweep" kernel per 8-bit
-// digit that ranks a tile with warp match/ballot, publishes per-digit tile counts through
-// decoupled look-back, and scatters through shared memory so that global writes go out
-// in digit runs.
+// one histogram pass over the keys for every digit, then one kernel per 8-bit digit that
+// ranks a tile with shared-memory counters, publishes per-digit tile counts through
+// decoupled look-back, and writes the tile out in digit runs.
 //
 // Keys are containers of K bytes (1..64), sorted on bits [begin_bit, end_bit) as
 // unsigned integers, values V bytes (0 = keys only).  The sort is stable, so it orders
@@ -11,6 +10,7 @@
 #pragma once
 
 #include "rfx_device.cuh"
+#include "tile_ring.cuh"
 
 namespace rfx {
 
@@ -18,21 +18,33 @@ constexpr int kSortThreads = 256;   // the histogram pass
 constexpr int kRadix = 256;
 constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kMaxSortPasses = 16;  // up to 128 key bits per call
-constexpr int kSortLookWindow = 8;  // predecessors examined per look-back round trip
+constexpr int kSortLookWindow = 8;  // predecessors examined per look-back round trip (16: 2 % slower, 32: 8 %)
 
-// Items per thread by the bytes moved per item: tiles of 24-48 KB (as large as 128
-// registers allow without spills), so the per-tile fixed costs (barriers, the look-back)
-// are spread over enough keys.
+// The tile of a digit pass by the bytes of a key and its value.  Two blocks per SM: as large
+// a tile as their shared memory allows (the per-tile costs -- barriers, the look-back -- and
+// the number of digit runs a tile is written in fall with its size), over as many threads as
+// that leaves registers for.  60M keys, us per pass, of the shapes tried:
+//   4 B   512 x 20 and 384 x 24: 212; 512 x 16, 384 x 16 with 3 blocks: 218; 512 x 12: 241
+//   8 B   384 x 16: 274; 512 x 12: 277; 512 x 8: 335
+//   16 B  512 x 8: 407; 384 x 10: 422; 1024 x 8, one block: 436
+//   4 B keys with 8 B values (4M): 384 x 12: 31.5; 512 x 8: 35.1; 512 x 12, one block: 37.6
 template <int K, int V>
 struct SortTuning {
   static constexpr int B = K + V;
-  // a digit pass: 8 warps per block for elements up to 8 bytes, 12 above (two blocks per SM
-  // either way; the larger elements' passes gain from the extra warps, the smaller lose)
-  static constexpr int THREADS = B <= 8 ? 256 : 384;
+  static constexpr int THREADS = B <= 4 ? 512 : B <= 12 ? 384 : B <= 16 ? 512 : B <= 48 ? 384 : 256;
+  static constexpr int IPT = B <= 4 ? 20 : B <= 8 ? 16 : B <= 12 ? 12 : B <= 16 ? 8 : B <= 32 ? 6 : 4;
   static constexpr int WARPS = THREADS / 32;
-  static constexpr int IPT = B <= 4 ? 24 : B <= 8 ? 20 : B <= 16 ? 8 : B <= 32 ? 5 : B <= 64 ? 3 : 1;
   static constexpr int TILE = THREADS * IPT;
-  static constexpr int SBYTES = (K > V ? K : V);
+  // dynamic shared memory: the tile's keys and values as they lie in global memory, every
+  // warp's digit counters, one 32-bit entry per element
+  static constexpr size_t KEYS = (size_t)TILE * K;
+  static constexpr size_t VALS = (size_t)TILE * V;
+  static constexpr size_t COUNTERS = (size_t)WARPS * 256 * 4;
+  static constexpr size_t SMEM = KEYS + VALS + COUNTERS + (size_t)TILE * 4;
+  static_assert(THREADS >= 256, "one thread per digit");
+  static_assert(TILE <= 0x10000, "an element's place in its tile fits 16 bits");
+  static_assert(KEYS % 16 == 0 && VALS % 16 == 0 && COUNTERS % 16 == 0, "16-byte aligned parts");
+  static_assert(2 * (SMEM + 4096) <= 228 * 1024, "two blocks per SM");
 };
 
 // A K-byte element as 32-bit words (1- and 2-byte elements zero-extended into w[0]).
@@ -129,14 +141,6 @@ __device__ __forceinline__ uint32_t ld_relaxed_u32(const uint32_t* p) {
   asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ uint4 ld_volatile_v4(const uint32_t* p) {
-  uint4 v;
-  asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p)
-               : "memory");
-  return v;
-}
 __device__ __forceinline__ void st_relaxed_u32(uint32_t* p, uint32_t v) {
   asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -218,253 +222,268 @@ sort_histogram_kernel(const uint8_t* __restrict__ keys, uint64_t n, uint32_t beg
   }
 }
 
-// ------------------------------------------------------------------ per-tile pass
-// Two blocks per SM: the per-item keys and ranks must fit 128 registers, so digits and
-// tile positions are recomputed where needed instead of being kept live.
+// ------------------------------------------------------------------ digit pass
+// Per tile:
+//   load     one thread copies the tile into shared memory by bulk copies (elements of
+//            arrays that are not 16-byte aligned, and the last elements of the last tile,
+//            by plain loads), after the previous tile has been written out;
+//   rank     every key takes the next count of its digit from its warp's counters by one
+//            shared-memory atomic add; the keys themselves stay where they are;
+//   count    per digit: the warps' counts become starts within the tile, the tile's count
+//            is published for the successors' look-back;
+//   order    every key's entry (digit << 16 | place in the tile) goes to its slot;
+//   prefix   the digits' global offsets, by decoupled look-back;
+//   write    the slots are written out in order, the keys read through their entries: one
+//            run of consecutive addresses per digit.
 //
-// A block claims its next tile one ahead and, where the keys are 16-byte aligned and two
-// tile buffers fit, copies that tile's keys into shared memory with cp.async while it
-// ranks, resolves and writes the current one, so the load of a tile never waits on the
-// memory system.  Per tile: rank in registers, count digits and publish the tile's
-// aggregate, scatter the keys into the tile's own buffer in digit order, resolve the
-// global digit offsets by decoupled look-back (after the scatter, so the predecessors
-// have had that long to publish), then write the buffer out in digit runs.
-template <int K, int V>
-struct SortBuffers {
-  static constexpr int EB = (int)sizeof(Elem<K>) > (V > 0 ? (int)sizeof(Elem<V>) : 0) ? (int)sizeof(Elem<K>)
-                                                                                        : (int)sizeof(Elem<V>);
-  static constexpr int TILE = SortTuning<K, V>::TILE;
-  // prefetch when the raw keys are whole 16-byte chunks and two buffers fit two blocks
-  static constexpr bool PF = K >= 4 && 2 * TILE * EB <= 100 * 1024;
-  static constexpr size_t SMEM = (size_t)(PF ? 2 : 1) * TILE * EB;
-};
+// What bounds it: shared-memory wavefronts (accesses by digit hit random banks) for narrow
+// keys, HBM for 16-byte ones.  The ranks were found by an atomic OR of the lane into a
+// per-digit mask, two reads, a count update and a clear before (29 wavefronts per 32 keys
+// in all, now about 20), and a tile was claimed one ahead of its turn: a claimed tile waits
+// for its block's current one, and every later tile's look-back waits for it, so all
+// blocks ran at the pace of the slowest.  A tile is now claimed while the one before it is
+// written out, and what a block will claim about a round later is brought into L2 by a
+// prefetch.  60M keys, us per pass, before -> now: 4 B 325 -> 212, 8 B 430 -> 274, 16 B 605 -> 407.
+//
+// Stability.  The order in which one atomic instruction serves the lanes that share a digit
+// is not specified, so the keys of one warp step may come out exchanged.  Entries must
+// ascend over the tile; the block looks at every neighbouring pair (read anyway for the
+// write-out) and, should any be out of order, sorts the entries by odd-even transposition.
+// Every exchange is between neighbouring slots, so that ends after a few rounds.
 
-// The raw keys of tile `tile` (tcount keys) into `dst`, in 16-byte chunks (the last one
-// zero-filled past the array).
+// The bits of element i of a raw shared-memory array from bit 32 * q + sh on, at least the
+// digit's; `straddle`: the digit reaches into the next word.
 template <int K>
-__device__ __forceinline__ void sort_prefetch(uint8_t* dst, const uint8_t* keys, uint64_t tile, uint32_t tile_keys,
-                                              uint64_t n, uint32_t nthreads) {
-  block_prefetch16(dst, keys, tile * (uint64_t)tile_keys * K, (uint64_t)tile_keys * K, n * K, nthreads);
-}
-
-// The lanes of a warp whose digit equals this lane's (within `valid`): the intersection
-// over the digit's bits of the ballot of lanes sharing that bit (lop3-friendly form), or
-// the hardware match.
-template <bool MATCH>
-__device__ __forceinline__ unsigned digit_peers(uint32_t d, bool valid, uint32_t bits) {
-  if constexpr (MATCH) {
-    const unsigned m = __match_any_sync(0xffffffffu, valid ? d : 0xffffffffu);
-    return valid ? m : 0u;
+__device__ __forceinline__ uint32_t raw_digit(const uint8_t* raw, uint32_t i, uint32_t q, uint32_t sh, bool straddle) {
+  if constexpr (K == 1) {
+    return raw[i] >> sh;
+  } else if constexpr (K == 2) {
+    return reinterpret_cast<const uint16_t*>(raw)[i] >> sh;
   } else {
-    unsigned peers = __ballot_sync(0xffffffffu, valid);
-#pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      if ((uint32_t)b < bits) {
-        const unsigned bb = __ballot_sync(0xffffffffu, (d >> b) & 1u);
-        const unsigned mb = 0u - ((d >> b) & 1u);   // all ones where this lane's bit is set
-        peers &= ~(bb ^ mb);
-      }
-    }
-    return peers;
+    const uint32_t* p = reinterpret_cast<const uint32_t*>(raw) + i * (K / 4) + q;
+    if (!straddle) return p[0] >> sh;
+    return __funnelshift_r(p[0], q + 1 < K / 4 ? p[1] : 0u, sh);
   }
 }
 
-template <int K, int V, bool MATCH = false>
+// The exclusive prefix of digit threadIdx.x over the tiles before `tile` (tile > 0): the
+// words of kSortLookWindow predecessors per round trip, taken up to the first inclusive or
+// missing one.
+__device__ __forceinline__ uint32_t sort_lookback(const uint32_t* status, uint32_t tile, uint32_t* err) {
+  uint32_t prefix = 0, spins = 0;
+  int32_t base = (int32_t)tile - 1;
+  while (base >= 0) {
+    uint32_t w[kSortLookWindow];
+    // predecessor base - r sits r * kRadix words below base's word: constant offsets from
+    // one pointer (a window reaching past tile 0 reads "inclusive 0" there)
+    const uint32_t* p = status + (uint64_t)base * kRadix + threadIdx.x;
+    if (base >= kSortLookWindow - 1) {
+#pragma unroll
+      for (int r = 0; r < kSortLookWindow; ++r) w[r] = ld_relaxed_u32(p - r * kRadix);
+    } else {
+#pragma unroll
+      for (int r = 0; r < kSortLookWindow; ++r) w[r] = r <= base ? ld_relaxed_u32(p - r * kRadix) : kSFlagInc;
+    }
+    bool open = true, done = false;
+    uint32_t used = 0;
+#pragma unroll
+    for (int r = 0; r < kSortLookWindow; ++r) {
+      if (open && w[r] != 0) {
+        prefix += w[r] & kSValMask;
+        ++used;
+        done = (w[r] & kSFlagInc) != 0;
+      }
+      open = open && w[r] != 0 && !done;
+    }
+    if (done) break;
+    base -= (int32_t)used;
+    if (used == 0) {
+      if (++spins > kSpinLimit) {
+        raise_error(err, kErrTimeout);
+        break;
+      }
+      if (spins > 4) __nanosleep(spins < 16 ? 20 : 128);
+    }
+  }
+  return prefix;
+}
+
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
+template <int K, int V>
 __global__ void __launch_bounds__((SortTuning<K, V>::THREADS), 2)
 sort_pass_kernel(const SortPassArgs a) {
   using T = SortTuning<K, V>;
-  using SB = SortBuffers<K, V>;
-  constexpr int IPT = T::IPT;
-  constexpr int TILE = T::TILE;
-  extern __shared__ __align__(16) uint8_t sbuf[];              // 1 or 2 buffers of TILE * EB
-  __shared__ uint16_t whist[T::WARPS][kRadix];               // per-warp digit counts (a tile's fit 16 bits)
-  __shared__ uint32_t s_local[kRadix];                         // tile-local digit start
-  __shared__ unsigned long long s_gb[kRadix];                  // output index of slot i = s_gb[digit] + i
-  __shared__ uint8_t s_dig[TILE];                              // digit of each sorted slot
-  __shared__ uint32_t s_scan[T::WARPS];
-  __shared__ uint32_t s_tile[2];
+  constexpr int IPT = T::IPT, WARPS = T::WARPS;
+  constexpr uint32_t TILE = T::TILE, THREADS = T::THREADS;
+  extern __shared__ __align__(16) uint8_t sbuf[];
+  uint8_t* const raw = sbuf;
+  uint8_t* const rawv = sbuf + T::KEYS;
+  uint32_t* const counters = reinterpret_cast<uint32_t*>(sbuf + T::KEYS + T::VALS);
+  uint32_t* const entries = counters + T::COUNTERS / 4;
+  __shared__ uint32_t s_base[kRadix];   // output index of slot i = s_base[digit] + i (modulo 2^32)
+  __shared__ uint32_t s_scan[kRadix / 32];
+  __shared__ uint32_t s_tile;
+  __shared__ __align__(8) uint64_t s_bar;
   const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const uint64_t num_tiles = (a.n + TILE - 1) / TILE;
-  const bool pf = SB::PF && (reinterpret_cast<uintptr_t>(a.keys_in) & 15u) == 0;
-  const uint32_t dbits = 32 - __clz(a.mask);   // bits in this pass's digit (ballots needed)
-  if (t == 0) s_tile[0] = atomicAdd(a.tile_counter, 1u);
-  __syncthreads();
-  if (pf && s_tile[0] < num_tiles) sort_prefetch<K>(sbuf, a.keys_in, s_tile[0], TILE, a.n, T::THREADS);
-  cp_async_commit();
+  const uint32_t n = (uint32_t)a.n;   // below 2^30
+  const uint32_t num_tiles = (n + TILE - 1) / TILE;
+  const uint32_t q = a.shift >> 5, sh = a.shift & 31, mask = a.mask;
+  const bool straddle = sh + (32 - __clz(mask)) > 32;
+  const bool bulk =
+      ((reinterpret_cast<uintptr_t>(a.keys_in) | (V ? reinterpret_cast<uintptr_t>(a.vals_in) : 0u)) & 15u) == 0;
+  uint32_t* const wcount = counters + warp * kRadix;
+  const uint32_t gexcl = t < kRadix ? a.gexcl[t] : 0u;
 
-  for (uint32_t it = 0;; ++it) {
-    const uint64_t tile = s_tile[it & 1];
-    uint8_t* stage = sbuf + (pf ? (size_t)(it & 1) * TILE * SB::EB : 0);
-    if (t == 0) s_tile[(it + 1) & 1] = atomicAdd(a.tile_counter, 1u);   // the next tile, one ahead
-    for (uint32_t k = t; k < T::WARPS * kRadix / 2; k += T::THREADS) reinterpret_cast<uint32_t*>(&whist[0][0])[k] = 0;
-    __syncthreads();
-    if (tile >= num_tiles) break;   // the tile claimed next is larger still: no copy in flight
-    const uint64_t next = s_tile[(it + 1) & 1];
-    if (pf) {
-      if (next < num_tiles) sort_prefetch<K>(sbuf + (size_t)((it + 1) & 1) * TILE * SB::EB, a.keys_in, next, TILE, a.n, T::THREADS);
-      cp_async_commit();
-      cp_async_wait<1>();          // this tile's copy (the next one may stay in flight)
-      __syncthreads();
-    }
-    const uint64_t tbase = tile * TILE;
-    const uint32_t tcount = (uint32_t)min((uint64_t)TILE, a.n - tbase);
-    // warp w owns items [w*32*IPT, (w+1)*32*IPT) of the tile, item j of lane l at j*32+l
-    const uint32_t wbase = warp * 32 * IPT;
-    Elem<K> key[IPT];
-    uint32_t rank[IPT];
-#pragma unroll
-    for (int j = 0; j < IPT; ++j) {
-      const uint32_t li = wbase + j * 32 + lane;
-      if (li < tcount) key[j] = pf ? load_elem<K>(stage, li) : load_elem<K>(a.keys_in, tbase + li);
-    }
-    // the lanes of a warp whose key has this lane's digit: every key's bit goes into its
-    // digit's mask with one shared-memory atomic OR (the warp's 256 masks sit in the tile
-    // buffer, which is free from here until the scatter: every key is in registers), or the
-    // hardware match in the MATCH variant
-    uint32_t* s_peer = reinterpret_cast<uint32_t*>(stage) + warp * kRadix;
-    if constexpr (!MATCH) {
-      __syncthreads();   // all warps hold their keys
-      for (uint32_t k = lane; k < kRadix; k += 32) s_peer[k] = 0u;
-      __syncwarp();
-    }
-#pragma unroll
-    for (int j = 0; j < IPT; ++j) {
-      const uint32_t li = wbase + j * 32 + lane;
-      const bool valid = li < tcount;
-      const uint32_t d = valid ? (elem_bits<K>(key[j], a.shift) & a.mask) : 0u;
-      unsigned peers;
-      if constexpr (MATCH) {
-        peers = digit_peers<true>(d, valid, dbits);
-      } else {
-        if (valid) atomicOr(&s_peer[d], 1u << lane);
-        __syncwarp();
-        peers = valid ? s_peer[d] : 0u;
+  auto load = [&](uint32_t tile) {
+    const uint32_t base = tile * TILE, cnt = min(TILE, n - base);
+    uint32_t k0 = 0, v0 = 0;   // elements the bulk copies bring
+    if (bulk) {
+      const uint32_t kb = cnt * K & ~15u, vb = cnt * V & ~15u;
+      if (t == 0) {
+        fence_proxy_async_smem();   // the buffers were read and written by plain accesses
+        mbar_arrive_tx(&s_bar, kb + vb);
+        if (kb) bulk_copy_g2s(raw, a.keys_in + (uint64_t)base * K, kb, &s_bar);
+        if (vb) bulk_copy_g2s(rawv, a.vals_in + (uint64_t)base * V, vb, &s_bar);
       }
-      const unsigned lower = peers & ((1u << lane) - 1);
-      uint32_t base = 0;
-      if (valid) base = whist[warp][d];
-      rank[j] = (base + __popc(lower)) | (d << 16);   // the digit rides along: extracted once
-      __syncwarp();
-      if (valid && lower == 0) {
-        whist[warp][d] = (uint16_t)(base + __popc(peers));
-        if constexpr (!MATCH) s_peer[d] = 0u;   // cleared for the next key by its group's first lane
-      }
-      __syncwarp();
+      k0 = kb / K;
+      if constexpr (V > 0) v0 = vb / V;
+    }
+    for (uint32_t i = k0 + t; i < cnt; i += THREADS) store_elem<K>(raw, i, load_elem<K>(a.keys_in, (uint64_t)base + i));
+    if constexpr (V > 0)
+      for (uint32_t i = v0 + t; i < cnt; i += THREADS)
+        store_elem<V>(rawv, i, load_elem<V>(a.vals_in, (uint64_t)base + i));
+  };
+
+  if (t == 0) {
+    mbar_init(&s_bar, 1);
+    mbar_fence_init();
+    s_tile = atomicAdd(a.tile_counter, 1u);
+  }
+  for (uint32_t k = t; k < T::COUNTERS / 16; k += THREADS) reinterpret_cast<uint4*>(counters)[k] = make_uint4(0, 0, 0, 0);
+  __syncthreads();
+  uint32_t tile = s_tile;
+  if (tile < num_tiles) load(tile);
+  for (uint32_t parity = 0; tile < num_tiles; parity ^= 1u) {
+    const uint32_t tcount = min(TILE, n - tile * TILE);
+    const bool full = tcount == TILE;
+    if (!full || !bulk) __syncthreads();   // elements brought by plain loads
+    if (bulk && !mbar_wait(&s_bar, parity)) {
+      raise_error(a.err, kErrTimeout);
+      mbar_wait(&s_bar, parity);   // the copy is this block's own: no exit before it lands
+    }
+    // warp w owns elements [w * 32 * IPT, (w + 1) * 32 * IPT) of the tile, element j of lane l
+    // at j * 32 + l; the first nv of a lane's elements exist
+    const uint32_t first = warp * 32 * IPT + lane;
+    const uint32_t nv = first >= tcount ? 0u : (tcount - first + 31) / 32;
+    uint32_t digit[IPT], rank[IPT];
+#pragma unroll
+    for (int j = 0; j < IPT; ++j) digit[j] = raw_digit<K>(raw, first + j * 32, q, sh, straddle) & mask;
+    if (full) {
+#pragma unroll
+      for (int j = 0; j < IPT; ++j) rank[j] = atomicAdd(&wcount[digit[j]], 1u);
+    } else {
+#pragma unroll
+      for (int j = 0; j < IPT; ++j) rank[j] = (uint32_t)j < nv ? atomicAdd(&wcount[digit[j]], 1u) : 0u;
     }
     __syncthreads();
-    // per digit: exclusive over warps, the tile's count (published at once), tile-local start
-    uint32_t count = 0;
+    const uint32_t ahead = tile + gridDim.x;   // claimed by some block about a round from now
+    if (bulk && t == THREADS - 1 && ahead < num_tiles) {
+      const uint32_t ab = ahead * TILE, ac = min(TILE, n - ab), kb = ac * K & ~15u, vb = ac * V & ~15u;
+      if (kb) prefetch_l2(a.keys_in + (uint64_t)ab * K, kb);
+      if (vb) prefetch_l2(a.vals_in + (uint64_t)ab * V, vb);
+    }
+    // thread t < 256, digit t: the warps' counts as exclusive sums, the tile's count
+    // (published at once), the tile-local start
+    uint32_t before[WARPS], count = 0, start = 0;
+    uint32_t* const status = a.status + (uint64_t)tile * kRadix + t;
     if (t < kRadix) {
 #pragma unroll
-      for (int w = 0; w < T::WARPS; ++w) {
-        const uint32_t c = whist[w][t];
-        whist[w][t] = (uint16_t)count;
+      for (int w = 0; w < WARPS; ++w) before[w] = counters[w * kRadix + t];
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) {
+        const uint32_t c = before[w];
+        before[w] = count;
         count += c;
       }
-      st_relaxed_u32(a.status + tile * kRadix + t, (tile == 0 ? kSFlagInc : kSFlagAgg) | count);
-    }
-    // block exclusive scan of count over the 256 digits
-    uint32_t incl = count;
+      st_relaxed_u32(status, tile == 0 ? kSFlagInc | (gexcl + count) : kSFlagAgg | count);
+      uint32_t incl = count;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= (uint32_t)o) incl += v;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += v;
+      }
+      if (lane == 31) s_scan[warp] = incl;
+      start = incl - count;
     }
-    if (lane == 31) s_scan[warp] = incl;
     __syncthreads();
     if (t < kRadix) {
-      uint32_t wpre = 0;
-      for (uint32_t w = 0; w < warp; ++w) wpre += s_scan[w];
-      s_local[t] = wpre + incl - count;
+#pragma unroll
+      for (uint32_t w = 0; w < kRadix / 32; ++w) start += w < warp ? s_scan[w] : 0u;
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) counters[w * kRadix + t] = before[w] + start;
     }
     __syncthreads();
-    // keys: scatter into tile order in shared memory (every thread's keys are in registers),
-    // each slot's digit beside it
-    Elem<K>* skeys = reinterpret_cast<Elem<K>*>(stage);
+#pragma unroll
+    for (int j = 0; j < IPT; ++j)
+      if (full || (uint32_t)j < nv) entries[wcount[digit[j]] + rank[j]] = (digit[j] << 16) | (first + j * 32);
+    if (t < kRadix) {
+      uint32_t prefix = gexcl;
+      if (tile > 0) {
+        prefix = sort_lookback(a.status, tile, a.err);
+        st_relaxed_u32(status, kSFlagInc | ((prefix + count) & kSValMask));
+      }
+      s_base[t] = prefix - start;
+    }
+    __syncthreads();
+    for (uint32_t k = t; k < T::COUNTERS / 16; k += THREADS)
+      reinterpret_cast<uint4*>(counters)[k] = make_uint4(0, 0, 0, 0);
+    uint32_t entry[IPT];
+    bool disorder = false;
 #pragma unroll
     for (int j = 0; j < IPT; ++j) {
-      const uint32_t li = wbase + j * 32 + lane;
-      if (li < tcount) {
-        const uint32_t d = rank[j] >> 16;
-        const uint32_t slot = s_local[d] + whist[warp][d] + (rank[j] & 0xffffu);
-        skeys[slot] = key[j];
-        s_dig[slot] = (uint8_t)d;
-      }
+      const uint32_t i = j * THREADS + t;
+      entry[j] = entries[i];
+      disorder = disorder || (i > 0 && i < tcount && entries[i - 1] > entry[j]);
     }
-    // decoupled look-back for digit t, kSortLookWindow predecessors per round trip
-    // (independent loads, all in flight at once)
-    if (t < kRadix) {
-      uint32_t prefix = 0;
-      if (tile > 0) {
-        int64_t base = (int64_t)tile - 1;
-        uint32_t spins = 0;
-        while (base >= 0) {
-          uint32_t w[kSortLookWindow];
-          // predecessor base - r sits r * kRadix words below base's word: constant offsets
-          // from one pointer (a window reaching past tile 0 reads "inclusive 0" there)
-          const uint32_t* pb = a.status + (uint64_t)base * kRadix + t;
-          if (base >= kSortLookWindow - 1) {
-#pragma unroll
-            for (int r = 0; r < kSortLookWindow; ++r) w[r] = ld_relaxed_u32(pb - r * kRadix);
-          } else {
-#pragma unroll
-            for (int r = 0; r < kSortLookWindow; ++r) w[r] = r <= base ? ld_relaxed_u32(pb - r * kRadix) : kSFlagInc;
-          }
-          int r_inc = kSortLookWindow;
-#pragma unroll
-          for (int r = kSortLookWindow - 1; r >= 0; --r)
-            if (w[r] & kSFlagInc) r_inc = r;
-          bool busy = false;
-          uint32_t sum = 0;
-#pragma unroll
-          for (int r = 0; r < kSortLookWindow; ++r) {
-            if (r <= r_inc) {
-              busy = busy || (w[r] & ~kSValMask) == 0;
-              sum += w[r] & kSValMask;
+    if (__syncthreads_or(disorder)) {
+      bool more = true;
+      while (more) {
+        bool moved = false;
+        for (uint32_t odd = 0; odd < 2; ++odd) {
+          for (uint32_t i = 2 * t + odd; i + 1 < tcount; i += 2 * THREADS) {
+            const uint32_t x = entries[i], y = entries[i + 1];
+            if (x > y) {
+              entries[i] = y;
+              entries[i + 1] = x;
+              moved = true;
             }
           }
-          if (busy) {
-            if (++spins > kSpinLimit) {
-              raise_error(a.err, kErrTimeout);
-              break;
-            }
-            __nanosleep(spins < 16 ? 32 : 128);
-            continue;
-          }
-          prefix += sum;
-          if (r_inc < kSortLookWindow) break;
-          base -= kSortLookWindow;
+          __syncthreads();
         }
-        st_relaxed_u32(a.status + tile * kRadix + t, kSFlagInc | ((prefix + count) & kSValMask));
+        more = __syncthreads_or(moved);
       }
-      // (global start of the digit's run) - (its tile-local start), modulo 2^64
-      s_gb[t] = (unsigned long long)a.gexcl[t] + prefix - s_local[t];
-    }
-    __syncthreads();
-    for (uint32_t i = t; i < tcount; i += T::THREADS) {
-      const uint64_t pos = s_gb[s_dig[i]] + i;
-      if (pos < a.n) store_elem<K>(a.keys_out, pos, skeys[i]);
-    }
-    if constexpr (V > 0) {
-      __syncthreads();
-      Elem<V>* svals = reinterpret_cast<Elem<V>*>(stage);
 #pragma unroll
-      for (int j = 0; j < IPT; ++j) {
-        const uint32_t li = wbase + j * 32 + lane;
-        if (li < tcount) {
-          const uint32_t d = rank[j] >> 16;
-          svals[s_local[d] + whist[warp][d] + (rank[j] & 0xffffu)] = load_elem<V>(a.vals_in, tbase + li);
+      for (int j = 0; j < IPT; ++j) entry[j] = entries[j * THREADS + t];
+    }
+    if (t == 0) s_tile = atomicAdd(a.tile_counter, 1u);   // the round trip hides behind the write-out
+#pragma unroll
+    for (int j = 0; j < IPT; ++j) {
+      const uint32_t i = j * THREADS + t, li = entry[j] & 0xffffu;
+      if (full || i < tcount) {
+        const uint32_t pos = s_base[entry[j] >> 16] + i;
+        if (pos < n) {
+          store_elem<K>(a.keys_out, pos, load_elem<K>(raw, li));
+          if constexpr (V > 0) store_elem<V>(a.vals_out, pos, load_elem<V>(rawv, li));
         }
-      }
-      __syncthreads();
-      for (uint32_t i = t; i < tcount; i += T::THREADS) {
-        const uint64_t pos = s_gb[s_dig[i]] + i;
-        if (pos < a.n) store_elem<V>(a.vals_out, pos, svals[i]);
       }
     }
     __syncthreads();
+    tile = s_tile;
+    if (tile < num_tiles) load(tile);
   }
-  cp_async_wait<0>();
 }
 
 }  // namespace rfx

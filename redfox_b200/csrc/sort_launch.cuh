@@ -4,8 +4,6 @@
 
 #include "host_common.h"
 #include "sort_kernels.cuh"
-#include "sort_onesweep.cuh"
-#include "tune.h"
 
 namespace rfx {
 
@@ -36,23 +34,9 @@ struct SortPlan {
   bool in_alt;          // out: the sorted data ended in the alternate buffers
 };
 
-// Look-back status words are laid out per tile of the smallest tile any pass variant
-// uses, so every variant's tiles fit the same status area.
-template <int K, int V>
-constexpr int min_sort_tile() {
-  if constexpr (V == 0 && (K == 4 || K == 8 || K == 16)) {
-    constexpr int a = SortTuning<K, V>::TILE, b = OsTuning<K, OsIpt<K>::SMALL>::TILE;
-    constexpr int c = OsTuning<K, OsIpt<K>::DEF>::TILE, d = OsTuning<K, OsIpt<K>::ALT>::TILE;
-    constexpr int ab = a < b ? a : b, cd = c < d ? c : d;
-    return ab < cd ? ab : cd;
-  } else {
-    return SortTuning<K, V>::TILE;
-  }
-}
-
 template <int K, int V>
 uint64_t sort_tiles(uint64_t n) {
-  return (n + min_sort_tile<K, V>() - 1) / min_sort_tile<K, V>();
+  return (n + SortTuning<K, V>::TILE - 1) / SortTuning<K, V>::TILE;
 }
 
 template <int K, int V>
@@ -72,42 +56,10 @@ rfx_status run_sort_kv(SortPlan& s) {
     RFX_CUDA_TRY(cudaStreamSynchronize(s.stream));
     for (uint32_t p = 0; p < s.passes; ++p) triv[p] = s.host_trivial[p];
   }
-  // Pass variants: 0 = the per-tile pass (every width, values too; the next tile's keys
-  // prefetched into shared memory); 1 / 2 / 3 = the pipelined onesweep pass (TMA stages +
-  // a look-back warp, one block per SM) with its default / fewer / other items per thread,
-  // where it applies: keys without values in 4/8/16-byte containers on 16-byte aligned
-  // buffers; 4 = the per-tile pass ranking with __match_any_sync instead of bit ballots
-  // (same keys).  The autotuner may pick per size class.
-  const size_t tile_smem = SortBuffers<K, V>::SMEM;
-  RFX_CUDA_TRY(allow_smem((const void*)sort_pass_kernel<K, V>, tile_smem));
-  if constexpr (V == 0 && (K == 4 || K == 8 || K == 16))
-    RFX_CUDA_TRY(allow_smem((const void*)sort_pass_kernel<K, V, true>, tile_smem));
-  const int tile_grid = persistent_grid((const void*)sort_pass_kernel<K, V>, SortTuning<K, V>::THREADS, tile_smem,
-                                        s.tiles ? s.tiles : 1);
-  constexpr bool kOnesweep = V == 0 && (K == 4 || K == 8 || K == 16);
-  bool os_ok = false;
-  int os_grid[3] = {0, 0, 0};   // default, small, alternative tiles
-  if constexpr (kOnesweep) {
-    os_ok = ((reinterpret_cast<uintptr_t>(s.keys) | reinterpret_cast<uintptr_t>(s.alt_keys) |
-              reinterpret_cast<uintptr_t>(s.alt2_keys)) & 15u) == 0;
-    if (os_ok) {
-      auto prep = [&](const void* k, size_t smem, int tile, int* grid) -> rfx_status {
-        const uint64_t ot = (s.n + tile - 1) / tile;
-        if (ot > s.tiles) return RFX_ERR_INVALID;   // the status area holds s.tiles tiles
-        RFX_CUDA_TRY(allow_smem(k, smem));
-        *grid = persistent_grid(k, kOsThreads, smem, ot ? ot : 1);
-        return RFX_OK;
-      };
-      using TD = OsTuning<K, OsIpt<K>::DEF>;
-      using TS = OsTuning<K, OsIpt<K>::SMALL>;
-      using TL = OsTuning<K, OsIpt<K>::ALT>;
-      rfx_status st = prep((const void*)sort_onesweep_kernel<K, TD::IPT>, TD::SMEM, TD::TILE, &os_grid[0]);
-      if (st == RFX_OK) st = prep((const void*)sort_onesweep_kernel<K, TS::IPT>, TS::SMEM, TS::TILE, &os_grid[1]);
-      if (st == RFX_OK) st = prep((const void*)sort_onesweep_kernel<K, TL::IPT>, TL::SMEM, TL::TILE, &os_grid[2]);
-      if (st == RFX_ERR_INVALID) os_ok = false;   // not expected: the per-tile pass runs instead
-      else if (st != RFX_OK) return st;
-    }
-  }
+  auto pass = sort_pass_kernel<K, V>;
+  constexpr size_t smem = SortTuning<K, V>::SMEM;
+  RFX_CUDA_TRY(allow_smem((const void*)pass, smem));
+  const int grid = persistent_grid((const void*)pass, SortTuning<K, V>::THREADS, smem, s.tiles);
   // Buffers the passes go through: b[0] = keys, pass j reads b[j] and writes b[j + 1].
   // An even number of passes alternates keys / alt and ends in keys; an odd number >= 3
   // goes keys -> alt -> alt2 -> keys and then alternates, so it ends in keys too; a single
@@ -150,38 +102,8 @@ rfx_status run_sort_kv(SortPlan& s) {
     a.status = s.status + (uint64_t)p * s.tiles * kRadix;
     a.tile_counter = s.counters + p;
     a.err = s.err;
-    // a pass reads kin and writes kout only, so a candidate can run again (the tuner
-    // times each one); the look-back words and the tile counter are cleared between runs
-    bool fresh = true;
-    auto launch = [&](int v) -> rfx_status {
-      if (!fresh) {
-        RFX_CUDA_TRY(cudaMemsetAsync(a.status, 0, (size_t)s.tiles * kRadix * sizeof(uint32_t), s.stream));
-        RFX_CUDA_TRY(cudaMemsetAsync(a.tile_counter, 0, sizeof(uint32_t), s.stream));
-      }
-      fresh = false;
-      if constexpr (kOnesweep) {
-        using TD = OsTuning<K, OsIpt<K>::DEF>;
-        using TS = OsTuning<K, OsIpt<K>::SMALL>;
-        using TL = OsTuning<K, OsIpt<K>::ALT>;
-        if (v == 4)
-          sort_pass_kernel<K, V, true><<<tile_grid, SortTuning<K, V>::THREADS, tile_smem, s.stream>>>(a);
-        else if (os_ok && v == 1)
-          sort_onesweep_kernel<K, TD::IPT><<<os_grid[0], kOsThreads, TD::SMEM, s.stream>>>(a);
-        else if (os_ok && v == 2)
-          sort_onesweep_kernel<K, TS::IPT><<<os_grid[1], kOsThreads, TS::SMEM, s.stream>>>(a);
-        else if (os_ok && v == 3)
-          sort_onesweep_kernel<K, TL::IPT><<<os_grid[2], kOsThreads, TL::SMEM, s.stream>>>(a);
-        else
-          sort_pass_kernel<K, V><<<tile_grid, SortTuning<K, V>::THREADS, tile_smem, s.stream>>>(a);
-      } else {
-        sort_pass_kernel<K, V><<<tile_grid, SortTuning<K, V>::THREADS, tile_smem, s.stream>>>(a);
-      }
-      RFX_CUDA_TRY(cudaGetLastError());
-      return RFX_OK;
-    };
-    const int v = os_ok ? tune_pick(TUNE_SORT_PASS, (uint64_t)K << 8 | V, s.n, 5, launch, s.stream) : 0;
-    rfx_status st = launch(v);
-    if (st != RFX_OK) return st;
+    pass<<<grid, SortTuning<K, V>::THREADS, smem, s.stream>>>(a);
+    RFX_CUDA_TRY(cudaGetLastError());
     ++s.executed;
   }
   return RFX_OK;

@@ -213,3 +213,28 @@ def test_sort_from_all_trivial_and_overlap(cuda):
     st = R.LIB.rfx_sort_pairs_from(R._ptr(dk), None, R._ptr(dk[100:]), None, 4000, 4, 0, 0, 32, 0, R._ptr(s.ws), s.wsb,
                                    R._stream())
     assert st == R.ERR_INVALID
+
+
+# Keys per tile of the digit pass, by key and value bytes (SortTuning): 4 B 10240, up to 8 B
+# 6144, up to 12 B 4608, up to 16 B 4096, up to 32 B 2304, up to 48 B 1536, above 1024.
+TILE_KEYS = {(1, 0): 10240, (4, 0): 10240, (8, 0): 6144, (4, 4): 6144, (4, 8): 4608, (16, 0): 4096, (8, 8): 4096,
+             (16, 16): 2304, (32, 0): 2304, (32, 16): 1536, (64, 16): 1024}
+
+
+@pytest.mark.parametrize("kb,vb", sorted(TILE_KEYS))
+@pytest.mark.parametrize("extra", [-1, 0, 1, 2 * 10240 + 17])
+def test_sort_tile_edges_with_many_equal_digits(cuda, kb, vb, extra):
+    """One tile less a key, a whole tile, a key more, a few tiles; digits that straddle a
+    32-bit word and digits that most of a warp's keys share, whose order must stay."""
+    n = TILE_KEYS[kb, vb] + extra
+    keys = _keys(n, kb, seed=n + kb)
+    keys[:, (kb * 8 - 5) // 8] &= np.uint8(0x13)
+    vals = np.random.default_rng(n).integers(0, 256, (n, vb), dtype=np.uint8) if vb else None
+    for begin, end in ((0, min(kb * 8, 11)), (max(0, kb * 8 - 21), kb * 8 - 1)):
+        dk, dv = R.sorted_copy(_dev(keys, cuda), _dev(vals, cuda) if vb else None, begin_bit=begin, end_bit=end)
+        exp = O.sort_pairs(keys, vals, begin_bit=begin, end_bit=end) if vb else (O.sort_pairs(keys, begin_bit=begin,
+                                                                                              end_bit=end), None)
+        assert np.array_equal(to_np(dk), exp[0])
+        if vb:
+            assert np.array_equal(to_np(dv), exp[1])
+    assert R.device_status() == R.OK
