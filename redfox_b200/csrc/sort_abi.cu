@@ -49,7 +49,7 @@ struct SortLayout {
   uint8_t* alt2_vals;   // the caller's buffers instead of being copied back
   uint32_t* ctrl;  // ghist | trivial | done | counters
   uint32_t* status;
-  size_t ctrl_bytes;  // bytes to clear per chunk (ctrl + status)
+  size_t ctrl_bytes;  // bytes to clear per chunk (ctrl; the histogram clears status)
   size_t total;
   uint64_t tiles;
   uint32_t passes;
@@ -69,8 +69,8 @@ SortLayout layout(void* ws, uint64_t n, uint32_t kb, uint32_t vb, uint32_t begin
   c.used = align_up(c.used, 256);
   const size_t ctrl_start = c.used;
   L.ctrl = c.take<uint32_t>(kMaxSortPasses * kRadix + 2 * kMaxSortPasses + 1);
-  L.status = c.take<uint32_t>((size_t)L.passes * L.tiles * kRadix);
   L.ctrl_bytes = c.used - ctrl_start;
+  L.status = c.take<uint32_t>((size_t)L.passes * L.tiles * kRadix);
   L.total = align_up(c.used, 256);
   return L;
 }

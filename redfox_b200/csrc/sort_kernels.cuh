@@ -14,9 +14,7 @@
 
 namespace rfx {
 
-constexpr int kSortThreads = 256;   // the histogram pass
 constexpr int kRadix = 256;
-constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kMaxSortPasses = 16;  // up to 128 key bits per call
 constexpr int kSortLookWindow = 8;  // predecessors examined per look-back round trip (16: 2 % slower, 32: 8 %)
 
@@ -146,53 +144,119 @@ __device__ __forceinline__ void st_relaxed_u32(uint32_t* p, uint32_t v) {
 }
 
 // ------------------------------------------------------------------ histogram
-// Counts every pass's digits in one read of the keys (warp-aggregated shared atomics),
-// then the last block turns the counts into exclusive offsets and flags trivial passes.
-template <int K>
-__global__ void __launch_bounds__(kSortThreads)
-sort_histogram_kernel(const uint8_t* __restrict__ keys, uint64_t n, uint32_t begin_bit, uint32_t end_bit,
-                      uint32_t passes, uint32_t* __restrict__ ghist, uint32_t* __restrict__ trivial,
-                      uint32_t* __restrict__ done_counter) {
-  __shared__ uint32_t h[kMaxSortPasses][kRadix];
-  __shared__ bool s_last;
-  const uint32_t t = threadIdx.x, lane = t & 31;
-  for (uint32_t k = t; k < passes * kRadix; k += kSortThreads) (&h[0][0])[k] = 0;
-  __syncthreads();
-  // R elements per thread per iteration, all loaded before any is counted (a read-only
-  // stream needs several loads in flight per thread to approach HBM bandwidth)
-  constexpr int R = K <= 16 ? 4 : 2;
-  const uint64_t stride = (uint64_t)gridDim.x * kSortThreads;
-  const uint64_t nround = (n + R * stride - 1) / (R * stride) * (R * stride);  // warps stay converged
-  for (uint64_t i0 = (uint64_t)blockIdx.x * kSortThreads + t; i0 < nround; i0 += R * stride) {
-    Elem<K> e[R];
+// Counts the digits of up to kHistPlaces passes in one read of the keys (more passes: one
+// read per kHistPlaces), then the last block turns the counts into exclusive offsets and
+// flags trivial passes.  Also clears the look-back words of every pass.
+//
+// Every lane counts in bins of its own (bin d of lane l at word d * 32 + l, so that the 32
+// lanes always hit 32 banks): a digit is two or three instructions and one wavefront,
+// whatever its distribution.  Bins shared by the block, with a warp vote that took digits
+// equal in all lanes together, were bound by instruction issue and bank conflicts: 60M
+// 4-byte keys with four digits 337 us, 60M 16-byte rows 483 us.  16 bytes per load and
+// thread, kHistLoads loads in flight.
+constexpr int kHistThreads = 1024;
+constexpr int kHistPlaces = 4;
+constexpr int kHistLoads = 4;
+constexpr uint32_t kHistPlaceBytes = kRadix * 32 * 4;
+
+template <int PLACE>
+__device__ __forceinline__ void hist_count(uint32_t at) {
+  asm volatile("red.shared.add.u32 [%0 + %1], 1;" ::"r"(at), "n"(PLACE * kHistPlaceBytes) : "memory");
+}
+
+template <int K, int P>
+struct HistDigits {
+  uint32_t shift[P];   // first bit of each place's digit (single words: the rotation that brings it to bit 7)
+  uint32_t mask[P];    // the digit's mask, at bit 7
+  uint32_t at;         // this lane's bin 0 of place 0
+  __device__ __forceinline__ HistDigits(uint32_t bins, uint32_t begin, uint32_t end) : at(bins + (threadIdx.x & 31) * 4) {
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const uint64_t i = i0 + (uint64_t)r * stride;
-      if (i < n) e[r] = load_elem<K>(keys, i);
-    }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const bool valid = i0 + (uint64_t)r * stride < n;
-      const unsigned vmask = __ballot_sync(0xffffffffu, valid);
-      for (uint32_t p = 0; p < passes; ++p) {
-        const uint32_t shift = begin_bit + 8 * p;
-        const uint32_t w = end_bit - shift < 8 ? end_bit - shift : 8;
-        const uint32_t d = valid ? (elem_bits<K>(e[r], shift) & ((1u << w) - 1)) : kRadix;
-        // a digit shared by the whole warp (constant high digits) is one add, not 32
-        // conflicting atomics; otherwise plain shared atomics
-        const uint32_t d0 = __shfl_sync(0xffffffffu, d, 0);
-        if (__all_sync(0xffffffffu, d == d0 || !valid) && vmask == 0xffffffffu) {
-          if (lane == 0) atomicAdd(&h[p][d0], 32u);
-        } else if (valid) {
-          atomicAdd(&h[p][d], 1u);
-        }
-      }
+    for (int p = 0; p < P; ++p) {
+      const uint32_t s = begin + 8 * p;
+      const uint32_t w = s >= end ? 0u : end - s < 8 ? end - s : 8u;   // places past the last pass: digit 0
+      shift[p] = Elem<K>::NW == 1 ? (s - 7) & 31 : min(s, 8u * K - 1);
+      mask[p] = ((1u << w) - 1) << 7;
     }
   }
-  __syncthreads();
-  for (uint32_t k = t; k < passes * kRadix; k += kSortThreads) {
-    const uint32_t c = (&h[0][0])[k];
-    if (c) atomicAdd(&ghist[k], c);
+  template <int PLACE = 0>
+  __device__ __forceinline__ void count(const Elem<K>& e) const {
+    if constexpr (PLACE < P) {
+      uint32_t x;
+      if constexpr (Elem<K>::NW == 1) x = __funnelshift_r(e.w[0], e.w[0], shift[PLACE]);
+      else x = elem_bits<K>(e, shift[PLACE]) << 7;
+      hist_count<PLACE>(at + (x & mask[PLACE]));
+      count<PLACE + 1>(e);
+    }
+  }
+};
+
+// The digits of the elements in one 16-byte chunk.
+template <int K, int P>
+__device__ __forceinline__ void hist_chunk(const HistDigits<K, P>& h, const uint4& v) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  if constexpr (K <= 4) {
+#pragma unroll
+    for (int k = 0; k < 16 / K; ++k) {
+      Elem<K> e;
+      e.w[0] = w[k * K / 4] >> (8 * (k * K % 4));
+      h.count(e);
+    }
+  } else if constexpr (K == 8) {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      Elem<8> e;
+      e.w[0] = w[2 * k];
+      e.w[1] = w[2 * k + 1];
+      h.count(e);
+    }
+  } else {
+    Elem<16> e;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) e.w[k] = w[k];
+    h.count(e);
+  }
+}
+
+template <int K, int P>
+__global__ void __launch_bounds__(kHistThreads)
+sort_histogram_kernel(const uint8_t* __restrict__ keys, uint64_t n, uint32_t begin_bit, uint32_t end_bit,
+                      uint32_t passes, uint32_t* __restrict__ ghist, uint32_t* __restrict__ trivial,
+                      uint32_t* __restrict__ done_counter, uint4* __restrict__ status, uint64_t status_chunks) {
+  extern __shared__ __align__(16) uint32_t bins[];   // [P][256][32]
+  __shared__ bool s_last;
+  const uint32_t t = threadIdx.x, lane = t & 31;
+  const uint64_t tid = (uint64_t)blockIdx.x * kHistThreads + t, stride = (uint64_t)gridDim.x * kHistThreads;
+  for (uint64_t k = tid; k < status_chunks; k += stride) status[k] = make_uint4(0, 0, 0, 0);
+  // whole 16-byte chunks where the elements tile them; the rest element by element
+  const bool vec = K <= 16 && (reinterpret_cast<uintptr_t>(keys) & 15u) == 0;
+  const uint64_t chunks = vec ? n * K / 16 : 0;
+  for (uint32_t p0 = 0; p0 < passes; p0 += P) {
+    for (uint32_t k = t; k < P * kHistPlaceBytes / 16; k += kHistThreads)
+      reinterpret_cast<uint4*>(bins)[k] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+    const HistDigits<K, P> h(smem_u32(bins), begin_bit + 8 * p0, end_bit);
+    if constexpr (K <= 16) {
+      const uint4* src = reinterpret_cast<const uint4*>(keys);
+      for (uint64_t c = tid; c < chunks; c += kHistLoads * stride) {
+        uint4 v[kHistLoads];
+#pragma unroll
+        for (int u = 0; u < kHistLoads; ++u)
+          if (c + u * stride < chunks) v[u] = __ldg(src + c + u * stride);
+#pragma unroll
+        for (int u = 0; u < kHistLoads; ++u)
+          if (c + u * stride < chunks) hist_chunk<K, P>(h, v[u]);
+      }
+    }
+    for (uint64_t i = chunks * 16 / K + tid; i < n; i += stride) h.count(load_elem<K>(keys, i));
+    __syncthreads();
+    // bin b of the group, its 32 lanes' counts read in a rotated order (one bank per thread)
+    for (uint32_t b = t; b < min((uint32_t)P, passes - p0) * kRadix; b += kHistThreads) {
+      uint32_t sum = 0;
+#pragma unroll 8
+      for (uint32_t l = 0; l < 32; ++l) sum += bins[b * 32 + ((l + t) & 31)];
+      if (sum) atomicAdd(&ghist[p0 * kRadix + b], sum);
+    }
+    __syncthreads();
   }
   __threadfence();
   __syncthreads();
@@ -201,8 +265,7 @@ sort_histogram_kernel(const uint8_t* __restrict__ keys, uint64_t n, uint32_t beg
   if (!s_last) return;
   __threadfence();
   // exclusive scan per pass (one warp per pass)
-  const uint32_t warp = t >> 5;
-  for (uint32_t p = warp; p < passes; p += kSortWarps) {
+  for (uint32_t p = t >> 5; p < passes; p += kHistThreads / 32) {
     uint32_t run = 0, maxc = 0;
     for (uint32_t d0 = 0; d0 < kRadix; d0 += 32) {
       const uint32_t c = atomicAdd(&ghist[p * kRadix + d0 + lane], 0u);

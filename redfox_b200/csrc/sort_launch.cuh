@@ -39,17 +39,28 @@ uint64_t sort_tiles(uint64_t n) {
   return (n + SortTuning<K, V>::TILE - 1) / SortTuning<K, V>::TILE;
 }
 
+// Histogram of every digit; clears the look-back words.
+template <int K, int P>
+rfx_status launch_histogram(SortPlan& s) {
+  auto k = sort_histogram_kernel<K, P>;
+  constexpr size_t smem = P * (size_t)kHistPlaceBytes;
+  RFX_CUDA_TRY(allow_smem((const void*)k, smem));
+  const uint64_t per_block = (uint64_t)kHistThreads * kHistLoads * 16;   // bytes of one round of loads
+  const int grid = persistent_grid((const void*)k, kHistThreads, smem, (s.n * K + per_block - 1) / per_block);
+  k<<<grid, kHistThreads, smem, s.stream>>>(s.src_keys ? s.src_keys : s.keys, s.n, s.begin_bit, s.end_bit, s.passes,
+                                            s.ghist, s.trivial, s.done, reinterpret_cast<uint4*>(s.status),
+                                            s.passes * s.tiles * (kRadix / 4));
+  RFX_CUDA_TRY(cudaGetLastError());
+  return RFX_OK;
+}
+
 template <int K, int V>
 rfx_status run_sort_kv(SortPlan& s) {
-  // histogram of every digit
-  {
-    auto hk = sort_histogram_kernel<K>;
-    const uint64_t blocks = (s.n + kSortThreads * 8 - 1) / (kSortThreads * 8);
-    const int grid = persistent_grid((const void*)hk, kSortThreads, 0, blocks ? blocks : 1);
-    hk<<<grid, kSortThreads, 0, s.stream>>>(s.src_keys ? s.src_keys : s.keys, s.n, s.begin_bit, s.end_bit, s.passes,
-                                            s.ghist, s.trivial, s.done);
-    RFX_CUDA_TRY(cudaGetLastError());
-  }
+  rfx_status hst = s.passes == 1   ? launch_histogram<K, 1>(s)
+                   : s.passes == 2 ? launch_histogram<K, 2>(s)
+                   : s.passes == 3 ? launch_histogram<K, 3>(s)
+                                   : launch_histogram<K, kHistPlaces>(s);
+  if (hst != RFX_OK) return hst;
   uint32_t triv[kMaxSortPasses] = {0};
   if (s.skip_trivial) {
     RFX_CUDA_TRY(cudaMemcpyAsync(s.host_trivial, s.trivial, s.passes * sizeof(uint32_t), cudaMemcpyDeviceToHost, s.stream));
