@@ -146,8 +146,8 @@ rfx_status rfx_filter_aggregate(const void* in, uint64_t n, const rfx_tuple* in_
                                 void* stream);
 
 /* ---------------------------------------------------------------- sort */
-/* Flag for rfx_sort_pairs: read the digit histogram back and skip digit passes whose
- * digit is constant over the input (synchronises the stream once per 128-bit chunk). */
+/* Flag of rfx_sort_pairs, accepted and without effect: digit passes whose digit is constant
+ * over the input are always skipped, on the device and without synchronising. */
 #define RFX_SORT_SKIP_TRIVIAL 1u
 
 /* Workspace of rfx_sort_pairs: the alternate key/value buffers plus histogram and

@@ -47,7 +47,7 @@ struct SortLayout {
   uint8_t* alt_vals;
   uint8_t* alt2_keys;   // with 3 or more digit passes: lets an odd number of passes end in
   uint8_t* alt2_vals;   // the caller's buffers instead of being copied back
-  uint32_t* ctrl;  // ghist | trivial | done | counters
+  uint32_t* ctrl;  // ghist | route | done | counters
   uint32_t* status;
   size_t ctrl_bytes;  // bytes to clear per chunk (ctrl; the histogram clears status)
   size_t total;
@@ -75,14 +75,11 @@ SortLayout layout(void* ws, uint64_t n, uint32_t kb, uint32_t vb, uint32_t begin
   return L;
 }
 
-thread_local uint32_t t_host_trivial[kMaxSortPasses];
-
 }  // namespace
 
 rfx_status sort_pairs_impl(void* keys, void* vals, uint64_t n, uint32_t kb, uint32_t vb, uint32_t begin_bit,
-                           uint32_t end_bit, void* ws, size_t ws_bytes, cudaStream_t stream, bool skip_trivial,
-                           int* passes_run, const void* src_keys = nullptr, const void* src_vals = nullptr) {
-  if (passes_run) *passes_run = 0;
+                           uint32_t end_bit, void* ws, size_t ws_bytes, cudaStream_t stream,
+                           const void* src_keys = nullptr, const void* src_vals = nullptr) {
   if (!valid_width(kb) || !valid_vwidth(vb)) return RFX_ERR_UNSUPPORTED;
   if (end_bit > kb * 8 || begin_bit > end_bit) return RFX_ERR_INVALID;
   if (src_keys && (n == 0 || !keys || (vb && (!vals || !src_vals)))) return n == 0 ? RFX_OK : RFX_ERR_INVALID;
@@ -138,24 +135,16 @@ rfx_status sort_pairs_impl(void* keys, void* vals, uint64_t n, uint32_t kb, uint
     s.end_bit = hi;
     s.passes = (hi - lo + 7) / 8;
     s.ghist = L.ctrl;
-    s.trivial = L.ctrl + kMaxSortPasses * kRadix;
-    s.done = s.trivial + kMaxSortPasses;
+    s.route = L.ctrl + kMaxSortPasses * kRadix;
+    s.done = s.route + kMaxSortPasses;
     s.counters = s.done + 1;
     s.status = L.status;
     s.tiles = L.tiles;
-    s.skip_trivial = skip_trivial;
-    s.host_trivial = t_host_trivial;
     s.err = err;
     s.stream = stream;
     rfx_status st = dispatch(kb, s, vb);
     if (st != RFX_OK) return st;
-    if (passes_run) *passes_run += s.executed;
-    if (from_src && s.executed == 0) {
-      // every pass was trivial: the output is a copy of the input
-      RFX_CUDA_TRY(cudaMemcpyAsync(cur_k, src_keys, n * kb, cudaMemcpyDeviceToDevice, stream));
-      if (vb) RFX_CUDA_TRY(cudaMemcpyAsync(cur_v, src_vals, n * vb, cudaMemcpyDeviceToDevice, stream));
-    }
-    if (s.in_alt) {
+    if (!from_src && s.passes == 1) {   // a single pass in place ends in the alternate buffers
       std::swap(cur_k, oth_k);
       std::swap(cur_v, oth_v);
     }
@@ -199,7 +188,7 @@ rfx_status sort_sync(void* keys, void* vals, uint64_t n, uint32_t kb, uint32_t v
   const size_t need = sort_workspace_impl(n, kb, vb, begin, end);
   void* ws = nullptr;
   RFX_CUDA_TRY(cudaMallocAsync(&ws, need, s));
-  rfx_status st = sort_pairs_impl(keys, vals, n, kb, vb, begin, end, ws, need, s, true, nullptr);
+  rfx_status st = sort_pairs_impl(keys, vals, n, kb, vb, begin, end, ws, need, s);
   cudaError_t e = cudaFreeAsync(ws, s);
   if (st != RFX_OK) return st;
   RFX_CUDA_TRY(e);
@@ -221,7 +210,7 @@ extern "C" rfx_status rfx_sort_pairs(void* keys, void* values, uint64_t n, uint3
                                      uint32_t begin_bit, uint32_t end_bit, uint32_t flags, void* workspace,
                                      size_t workspace_bytes, void* stream) {
   return sort_pairs_impl(keys, values, n, key_bytes, value_bytes, begin_bit, end_bit, workspace, workspace_bytes,
-                         as_stream(stream), (flags & RFX_SORT_SKIP_TRIVIAL) != 0, nullptr);
+                         as_stream(stream));
 }
 
 extern "C" rfx_status rfx_sort_pairs_from(const void* keys_in, const void* values_in, void* keys, void* values,
@@ -230,7 +219,7 @@ extern "C" rfx_status rfx_sort_pairs_from(const void* keys_in, const void* value
                                           void* stream) {
   if (n && !keys_in) return RFX_ERR_INVALID;
   return sort_pairs_impl(keys, values, n, key_bytes, value_bytes, begin_bit, end_bit, workspace, workspace_bytes,
-                         as_stream(stream), (flags & RFX_SORT_SKIP_TRIVIAL) != 0, nullptr, keys_in, values_in);
+                         as_stream(stream), keys_in, values_in);
 }
 
 extern "C" rfx_status rfx_b40c_sort_pair(void* keys, void* values, uint64_t n, uint64_t key_bits, uint64_t value_type) {

@@ -115,11 +115,45 @@ __device__ __forceinline__ uint32_t elem_bits(const Elem<K>& e, uint32_t shift) 
   }
 }
 
+// Where the passes read and write.  A pass whose digit is the same in every key moves
+// nothing; which passes those are is known on the device only (from the histogram), so the
+// histogram's last block plans the sequence and every pass kernel looks its part up:
+//   bits 0..1 source, 2..3 destination buffer (0 the source, 1 the output, 2 / 3 the
+//   alternates; in place 0 and 1 are the same), and what to do.
+constexpr uint32_t kRouteSort = 16;
+constexpr uint32_t kRouteCopy = 32;
+
+__device__ constexpr uint32_t sort_route(uint32_t what, uint32_t from, uint32_t to) {
+  return what | from | to << 2;
+}
+
+// The part of pass p of `passes`; bit p of `moving`: pass p's digits are not all the same.
+// The result ends in buffer 1, but for a single pass in place, which ends in 2 (the caller
+// copies it back; it always runs).  An even number of passes that move keys goes back and
+// forth between 1 and 2; in place an odd number from 3 on takes 2, 3, 1 first; a single one
+// is copied, before or after, by a pass that moves nothing itself.
+__device__ __forceinline__ uint32_t sort_plan(uint32_t moving, uint32_t passes, bool in_place, uint32_t p) {
+  if (passes == 1) moving = 1;
+  const uint32_t m = __popc(moving), last = 31 - __clz(moving);
+  if (m == 0) return !in_place && p == passes - 1 ? sort_route(kRouteCopy, 0, 1) : 0u;
+  if (in_place && m == 1 && passes > 1) {
+    if (last < passes - 1)
+      return p == last ? sort_route(kRouteSort, 0, 2) : p == passes - 1 ? sort_route(kRouteCopy, 2, 1) : 0u;
+    return p == last ? sort_route(kRouteSort, 2, 1) : p == 0 ? sort_route(kRouteCopy, 0, 2) : 0u;
+  }
+  if (!(moving >> p & 1)) return 0;
+  auto to = [&](uint32_t j) -> uint32_t {   // of the j-th pass that moves
+    if (!in_place || m % 2 == 0) return (m - 1 - j) % 2 ? 2 : 1;
+    return j == 1 ? 3 : j == 0 || j % 2 ? 2 : 1;
+  };
+  const uint32_t j = __popc(moving & ((1u << p) - 1));
+  return sort_route(kRouteSort, j ? to(j - 1) : 0u, to(j));
+}
+
 struct SortPassArgs {
-  const uint8_t* keys_in;
-  uint8_t* keys_out;
-  const uint8_t* vals_in;
-  uint8_t* vals_out;
+  uint8_t* keys[4];     // the buffers of the routes (keys[0] is only read when it is not keys[1])
+  uint8_t* vals[4];
+  const uint32_t* route;  // this pass's part
   uint64_t n;
   uint32_t shift;       // first bit of this digit
   uint32_t mask;        // digit mask (0xff, or fewer bits for the last digit)
@@ -146,7 +180,7 @@ __device__ __forceinline__ void st_relaxed_u32(uint32_t* p, uint32_t v) {
 // ------------------------------------------------------------------ histogram
 // Counts the digits of up to kHistPlaces passes in one read of the keys (more passes: one
 // read per kHistPlaces), then the last block turns the counts into exclusive offsets and
-// flags trivial passes.  Also clears the look-back words of every pass.
+// plans the passes (sort_plan).  Also clears the look-back words of every pass.
 //
 // Every lane counts in bins of its own (bin d of lane l at word d * 32 + l, so that the 32
 // lanes always hit 32 banks): a digit is two or three instructions and one wavefront,
@@ -220,10 +254,11 @@ __device__ __forceinline__ void hist_chunk(const HistDigits<K, P>& h, const uint
 template <int K, int P>
 __global__ void __launch_bounds__(kHistThreads)
 sort_histogram_kernel(const uint8_t* __restrict__ keys, uint64_t n, uint32_t begin_bit, uint32_t end_bit,
-                      uint32_t passes, uint32_t* __restrict__ ghist, uint32_t* __restrict__ trivial,
+                      uint32_t passes, uint32_t* __restrict__ ghist, uint32_t* __restrict__ route, bool in_place,
                       uint32_t* __restrict__ done_counter, uint4* __restrict__ status, uint64_t status_chunks) {
   extern __shared__ __align__(16) uint32_t bins[];   // [P][256][32]
   __shared__ bool s_last;
+  __shared__ uint32_t s_moving;   // bit p: pass p has more than one digit
   const uint32_t t = threadIdx.x, lane = t & 31;
   const uint64_t tid = (uint64_t)blockIdx.x * kHistThreads + t, stride = (uint64_t)gridDim.x * kHistThreads;
   for (uint64_t k = tid; k < status_chunks; k += stride) status[k] = make_uint4(0, 0, 0, 0);
@@ -264,11 +299,16 @@ sort_histogram_kernel(const uint8_t* __restrict__ keys, uint64_t n, uint32_t beg
   __syncthreads();
   if (!s_last) return;
   __threadfence();
+  if (t == 0) s_moving = 0;
+  __syncthreads();
   // exclusive scan per pass (one warp per pass)
   for (uint32_t p = t >> 5; p < passes; p += kHistThreads / 32) {
-    uint32_t run = 0, maxc = 0;
-    for (uint32_t d0 = 0; d0 < kRadix; d0 += 32) {
-      const uint32_t c = atomicAdd(&ghist[p * kRadix + d0 + lane], 0u);
+    uint32_t run = 0, maxc = 0, cnt[kRadix / 32];
+#pragma unroll
+    for (int r = 0; r < kRadix / 32; ++r) cnt[r] = ld_relaxed_u32(&ghist[p * kRadix + r * 32 + lane]);
+#pragma unroll
+    for (int r = 0; r < kRadix / 32; ++r) {
+      const uint32_t c = cnt[r], d0 = r * 32;
       maxc = max(maxc, c);
       uint32_t incl = c;
 #pragma unroll
@@ -281,8 +321,10 @@ sort_histogram_kernel(const uint8_t* __restrict__ keys, uint64_t n, uint32_t beg
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) maxc = max(maxc, __shfl_xor_sync(0xffffffffu, maxc, o));
-    if (lane == 0) trivial[p] = (uint64_t)maxc == n ? 1u : 0u;
+    if (lane == 0 && maxc != (uint32_t)n) atomicOr(&s_moving, 1u << p);
   }
+  __syncthreads();
+  if (t < passes) route[t] = sort_plan(s_moving, passes, in_place, t);
 }
 
 // ------------------------------------------------------------------ digit pass
@@ -375,9 +417,20 @@ __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
+// All n elements of B bytes from `src` to `dst`, by the whole grid.
+template <int B>
+__device__ void grid_copy(uint8_t* dst, const uint8_t* src, uint64_t n) {
+  const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+  const bool vec = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0;
+  const uint64_t chunks = vec ? n * B / 16 : 0;
+  for (uint64_t c = tid; c < chunks; c += stride)
+    reinterpret_cast<uint4*>(dst)[c] = reinterpret_cast<const uint4*>(src)[c];
+  for (uint64_t i = chunks * 16 / B + tid; i < n; i += stride) store_elem<B>(dst, i, load_elem<B>(src, i));
+}
+
 template <int K, int V>
 __global__ void __launch_bounds__((SortTuning<K, V>::THREADS), 2)
-sort_pass_kernel(const SortPassArgs a) {
+sort_pass_kernel(const __grid_constant__ SortPassArgs a) {
   using T = SortTuning<K, V>;
   constexpr int IPT = T::IPT, WARPS = T::WARPS;
   constexpr uint32_t TILE = T::TILE, THREADS = T::THREADS;
@@ -391,14 +444,34 @@ sort_pass_kernel(const SortPassArgs a) {
   __shared__ uint32_t s_tile;
   __shared__ __align__(8) uint64_t s_bar;
   const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const uint32_t route = *a.route;
   const uint32_t n = (uint32_t)a.n;   // below 2^30
   const uint32_t num_tiles = (n + TILE - 1) / TILE;
   const uint32_t q = a.shift >> 5, sh = a.shift & 31, mask = a.mask;
   const bool straddle = sh + (32 - __clz(mask)) > 32;
-  const bool bulk =
-      ((reinterpret_cast<uintptr_t>(a.keys_in) | (V ? reinterpret_cast<uintptr_t>(a.vals_in) : 0u)) & 15u) == 0;
   uint32_t* const wcount = counters + warp * kRadix;
   const uint32_t gexcl = t < kRadix ? a.gexcl[t] : 0u;
+  // a tile is claimed (and the counters cleared) while the route is on its way; a pass that
+  // turns out not to sort has no use for its tile numbers
+  if (t == 0) {
+    mbar_init(&s_bar, 1);
+    mbar_fence_init();
+    s_tile = atomicAdd(a.tile_counter, 1u);
+  }
+  for (uint32_t k = t; k < T::COUNTERS / 16; k += THREADS) reinterpret_cast<uint4*>(counters)[k] = make_uint4(0, 0, 0, 0);
+  __syncthreads();
+  // the buffers are looked up in the parameters where they are used, which leaves no register
+  // to their addresses
+  const uint32_t from = route & 3, to = route >> 2 & 3;
+  if (!(route & kRouteSort)) {
+    if (route & kRouteCopy) {
+      grid_copy<K>(a.keys[to], a.keys[from], a.n);
+      if constexpr (V > 0) grid_copy<V>(a.vals[to], a.vals[from], a.n);
+    }
+    return;
+  }
+  const bool bulk =
+      ((reinterpret_cast<uintptr_t>(a.keys[from]) | (V ? reinterpret_cast<uintptr_t>(a.vals[from]) : 0u)) & 15u) == 0;
 
   auto load = [&](uint32_t tile) {
     const uint32_t base = tile * TILE, cnt = min(TILE, n - base);
@@ -408,25 +481,18 @@ sort_pass_kernel(const SortPassArgs a) {
       if (t == 0) {
         fence_proxy_async_smem();   // the buffers were read and written by plain accesses
         mbar_arrive_tx(&s_bar, kb + vb);
-        if (kb) bulk_copy_g2s(raw, a.keys_in + (uint64_t)base * K, kb, &s_bar);
-        if (vb) bulk_copy_g2s(rawv, a.vals_in + (uint64_t)base * V, vb, &s_bar);
+        if (kb) bulk_copy_g2s(raw, a.keys[from] + (uint64_t)base * K, kb, &s_bar);
+        if (vb) bulk_copy_g2s(rawv, a.vals[from] + (uint64_t)base * V, vb, &s_bar);
       }
       k0 = kb / K;
       if constexpr (V > 0) v0 = vb / V;
     }
-    for (uint32_t i = k0 + t; i < cnt; i += THREADS) store_elem<K>(raw, i, load_elem<K>(a.keys_in, (uint64_t)base + i));
+    for (uint32_t i = k0 + t; i < cnt; i += THREADS) store_elem<K>(raw, i, load_elem<K>(a.keys[from], (uint64_t)base + i));
     if constexpr (V > 0)
       for (uint32_t i = v0 + t; i < cnt; i += THREADS)
-        store_elem<V>(rawv, i, load_elem<V>(a.vals_in, (uint64_t)base + i));
+        store_elem<V>(rawv, i, load_elem<V>(a.vals[from], (uint64_t)base + i));
   };
 
-  if (t == 0) {
-    mbar_init(&s_bar, 1);
-    mbar_fence_init();
-    s_tile = atomicAdd(a.tile_counter, 1u);
-  }
-  for (uint32_t k = t; k < T::COUNTERS / 16; k += THREADS) reinterpret_cast<uint4*>(counters)[k] = make_uint4(0, 0, 0, 0);
-  __syncthreads();
   uint32_t tile = s_tile;
   if (tile < num_tiles) load(tile);
   for (uint32_t parity = 0; tile < num_tiles; parity ^= 1u) {
@@ -441,22 +507,23 @@ sort_pass_kernel(const SortPassArgs a) {
     // at j * 32 + l; the first nv of a lane's elements exist
     const uint32_t first = warp * 32 * IPT + lane;
     const uint32_t nv = first >= tcount ? 0u : (tcount - first + 31) / 32;
-    uint32_t digit[IPT], rank[IPT];
+    uint32_t key[IPT];   // digit << 16 | rank among the warp's keys of that digit
 #pragma unroll
-    for (int j = 0; j < IPT; ++j) digit[j] = raw_digit<K>(raw, first + j * 32, q, sh, straddle) & mask;
+    for (int j = 0; j < IPT; ++j) key[j] = raw_digit<K>(raw, first + j * 32, q, sh, straddle) & mask;
     if (full) {
 #pragma unroll
-      for (int j = 0; j < IPT; ++j) rank[j] = atomicAdd(&wcount[digit[j]], 1u);
+      for (int j = 0; j < IPT; ++j) key[j] = key[j] << 16 | atomicAdd(&wcount[key[j]], 1u);
     } else {
 #pragma unroll
-      for (int j = 0; j < IPT; ++j) rank[j] = (uint32_t)j < nv ? atomicAdd(&wcount[digit[j]], 1u) : 0u;
+      for (int j = 0; j < IPT; ++j)
+        if ((uint32_t)j < nv) key[j] = key[j] << 16 | atomicAdd(&wcount[key[j]], 1u);
     }
     __syncthreads();
     const uint32_t ahead = tile + gridDim.x;   // claimed by some block about a round from now
     if (bulk && t == THREADS - 1 && ahead < num_tiles) {
       const uint32_t ab = ahead * TILE, ac = min(TILE, n - ab), kb = ac * K & ~15u, vb = ac * V & ~15u;
-      if (kb) prefetch_l2(a.keys_in + (uint64_t)ab * K, kb);
-      if (vb) prefetch_l2(a.vals_in + (uint64_t)ab * V, vb);
+      if (kb) prefetch_l2(a.keys[from] + (uint64_t)ab * K, kb);
+      if (vb) prefetch_l2(a.vals[from] + (uint64_t)ab * V, vb);
     }
     // thread t < 256, digit t: the warps' counts as exclusive sums, the tile's count
     // (published at once), the tile-local start
@@ -491,7 +558,8 @@ sort_pass_kernel(const SortPassArgs a) {
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < IPT; ++j)
-      if (full || (uint32_t)j < nv) entries[wcount[digit[j]] + rank[j]] = (digit[j] << 16) | (first + j * 32);
+      if (full || (uint32_t)j < nv)
+        entries[wcount[key[j] >> 16] + (key[j] & 0xffffu)] = (key[j] & 0xffff0000u) | (first + j * 32);
     if (t < kRadix) {
       uint32_t prefix = gexcl;
       if (tile > 0) {
@@ -538,8 +606,8 @@ sort_pass_kernel(const SortPassArgs a) {
       if (full || i < tcount) {
         const uint32_t pos = s_base[entry[j] >> 16] + i;
         if (pos < n) {
-          store_elem<K>(a.keys_out, pos, load_elem<K>(raw, li));
-          if constexpr (V > 0) store_elem<V>(a.vals_out, pos, load_elem<V>(rawv, li));
+          store_elem<K>(a.keys[to], pos, load_elem<K>(raw, li));
+          if constexpr (V > 0) store_elem<V>(a.vals[to], pos, load_elem<V>(rawv, li));
         }
       }
     }

@@ -10,28 +10,24 @@ namespace rfx {
 struct SortPlan {
   uint8_t* keys;
   uint8_t* vals;
-  const uint8_t* src_keys;   // when set, the first pass and the histogram read these instead
-  const uint8_t* src_vals;   // of keys / vals, which then only receive (out-of-place sort)
+  const uint8_t* src_keys;   // when set, the sort reads these and leaves them (out of place)
+  const uint8_t* src_vals;
   uint8_t* alt_keys;
   uint8_t* alt_vals;
-  uint8_t* alt2_keys;   // a second pair of alternate buffers (may be null): an odd number
-  uint8_t* alt2_vals;   // of passes >= 3 then ends in keys / vals without a copy
+  uint8_t* alt2_keys;   // a second pair of alternate buffers, with 3 or more passes
+  uint8_t* alt2_vals;
   uint64_t n;
   uint32_t begin_bit;
   uint32_t end_bit;     // end_bit - begin_bit <= 128
   uint32_t passes;
   uint32_t* ghist;      // [passes][256]
-  uint32_t* trivial;    // [passes]
+  uint32_t* route;      // [passes]
   uint32_t* done;       // 1
   uint32_t* counters;   // [passes]
   uint32_t* status;     // [passes][tiles][256]
   uint64_t tiles;
-  bool skip_trivial;
-  uint32_t* host_trivial;  // pinned or pageable host copy for skip_trivial
   uint32_t* err;
   cudaStream_t stream;
-  int executed;         // out: passes run
-  bool in_alt;          // out: the sorted data ended in the alternate buffers
 };
 
 template <int K, int V>
@@ -48,7 +44,7 @@ rfx_status launch_histogram(SortPlan& s) {
   const uint64_t per_block = (uint64_t)kHistThreads * kHistLoads * 16;   // bytes of one round of loads
   const int grid = persistent_grid((const void*)k, kHistThreads, smem, (s.n * K + per_block - 1) / per_block);
   k<<<grid, kHistThreads, smem, s.stream>>>(s.src_keys ? s.src_keys : s.keys, s.n, s.begin_bit, s.end_bit, s.passes,
-                                            s.ghist, s.trivial, s.done, reinterpret_cast<uint4*>(s.status),
+                                            s.ghist, s.route, !s.src_keys, s.done, reinterpret_cast<uint4*>(s.status),
                                             s.passes * s.tiles * (kRadix / 4));
   RFX_CUDA_TRY(cudaGetLastError());
   return RFX_OK;
@@ -61,50 +57,21 @@ rfx_status run_sort_kv(SortPlan& s) {
                    : s.passes == 3 ? launch_histogram<K, 3>(s)
                                    : launch_histogram<K, kHistPlaces>(s);
   if (hst != RFX_OK) return hst;
-  uint32_t triv[kMaxSortPasses] = {0};
-  if (s.skip_trivial) {
-    RFX_CUDA_TRY(cudaMemcpyAsync(s.host_trivial, s.trivial, s.passes * sizeof(uint32_t), cudaMemcpyDeviceToHost, s.stream));
-    RFX_CUDA_TRY(cudaStreamSynchronize(s.stream));
-    for (uint32_t p = 0; p < s.passes; ++p) triv[p] = s.host_trivial[p];
-  }
   auto pass = sort_pass_kernel<K, V>;
   constexpr size_t smem = SortTuning<K, V>::SMEM;
   RFX_CUDA_TRY(allow_smem((const void*)pass, smem));
   const int grid = persistent_grid((const void*)pass, SortTuning<K, V>::THREADS, smem, s.tiles);
-  // Buffers the passes go through: b[0] = keys, pass j reads b[j] and writes b[j + 1].
-  // An even number of passes alternates keys / alt and ends in keys; an odd number >= 3
-  // goes keys -> alt -> alt2 -> keys and then alternates, so it ends in keys too; a single
-  // pass (or no second buffer) ends in alt, which the caller copies back.
-  uint32_t npass = 0;
-  for (uint32_t p = 0; p < s.passes; ++p) npass += triv[p] ? 0u : 1u;
-  uint8_t* kb[kMaxSortPasses + 1];
-  uint8_t* vb[kMaxSortPasses + 1];
-  const bool three = (npass % 2 == 1) && npass >= 3 && s.alt2_keys && (V == 0 || s.alt2_vals);
-  for (uint32_t j = 0; j <= npass; ++j) {
-    const bool at_keys = three ? (j == 0 || (j >= 3 && j % 2 == 1)) : (j % 2 == 0);
-    const bool at_alt2 = three && j == 2;
-    kb[j] = at_keys ? s.keys : at_alt2 ? s.alt2_keys : s.alt_keys;
-    vb[j] = at_keys ? s.vals : at_alt2 ? s.alt2_vals : s.alt_vals;
-  }
-  if (s.src_keys) {
-    // out of place: the first pass reads the source (never written); a single pass writes
-    // straight into keys / vals
-    kb[0] = const_cast<uint8_t*>(s.src_keys);
-    vb[0] = const_cast<uint8_t*>(s.src_vals);
-    if (npass == 1) {
-      kb[1] = s.keys;
-      vb[1] = s.vals;
-    }
-  }
-  s.executed = 0;
-  s.in_alt = npass ? kb[npass] != s.keys : false;   // no pass at all: the data is where it was
   for (uint32_t p = 0; p < s.passes; ++p) {
-    if (triv[p]) continue;
     SortPassArgs a;
-    a.keys_in = kb[s.executed];
-    a.keys_out = kb[s.executed + 1];
-    a.vals_in = vb[s.executed];
-    a.vals_out = vb[s.executed + 1];
+    a.keys[0] = s.src_keys ? const_cast<uint8_t*>(s.src_keys) : s.keys;   // out of place: never written
+    a.vals[0] = s.src_keys ? const_cast<uint8_t*>(s.src_vals) : s.vals;
+    a.keys[1] = s.keys;
+    a.vals[1] = s.vals;
+    a.keys[2] = s.alt_keys;
+    a.vals[2] = s.alt_vals;
+    a.keys[3] = s.alt2_keys;
+    a.vals[3] = s.alt2_vals;
+    a.route = s.route + p;
     a.n = s.n;
     a.shift = s.begin_bit + 8 * p;
     const uint32_t w = s.end_bit - a.shift < 8 ? s.end_bit - a.shift : 8;
@@ -115,7 +82,6 @@ rfx_status run_sort_kv(SortPlan& s) {
     a.err = s.err;
     pass<<<grid, SortTuning<K, V>::THREADS, smem, s.stream>>>(a);
     RFX_CUDA_TRY(cudaGetLastError());
-    ++s.executed;
   }
   return RFX_OK;
 }

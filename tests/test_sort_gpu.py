@@ -238,3 +238,28 @@ def test_sort_tile_edges_with_many_equal_digits(cuda, kb, vb, extra):
         if vb:
             assert np.array_equal(to_np(dv), exp[1])
     assert R.device_status() == R.OK
+
+
+@pytest.mark.parametrize("moving", [[], [0], [1], [3], [0, 3], [0, 1, 2], [1, 2, 3], [0, 1, 2, 3]])
+@pytest.mark.parametrize("kb,vb,n", [(4, 0, 20_011), (8, 4, 9_001), (16, 0, 70_001)])
+def test_sort_skips_constant_digits_on_the_device(cuda, kb, vb, n, moving):
+    """Constant digits in every place among four: in place and out of place, keys and values."""
+    keys = np.full((n, kb), 0x5A, np.uint8)
+    rng = np.random.default_rng(n + sum(moving))
+    for b in moving:
+        keys[:, kb - 4 + b] = rng.integers(0, 256, n, dtype=np.uint8)
+    if kb > 4:
+        keys[:, 0] = rng.integers(0, 256, n, dtype=np.uint8)   # payload: shows the order of equal keys
+    vals = rng.integers(0, 256, (n, vb), dtype=np.uint8) if vb else None
+    begin, end = (kb - 4) * 8, kb * 8
+    exp = O.sort_pairs(keys, vals, begin_bit=begin, end_bit=end) if vb else (O.sort_pairs(keys, begin_bit=begin,
+                                                                                          end_bit=end), None)
+    a, av = _dev(keys, cuda), _dev(vals, cuda) if vb else None
+    b, bv = R.sorted_copy(a, av, begin_bit=begin, end_bit=end)
+    assert np.array_equal(to_np(a), keys)
+    R.sort_pairs(a, av, begin_bit=begin, end_bit=end)
+    for k, v in ((a, av), (b, bv)):
+        assert np.array_equal(to_np(k), exp[0])
+        if vb:
+            assert np.array_equal(to_np(v), exp[1])
+    assert R.device_status() == R.OK
