@@ -101,6 +101,56 @@ int persistent_grid(const void* kernel, int threads, size_t dyn_smem, uint64_t w
 }
 
 namespace {
+struct ClusterKey {
+  int dev;
+  const void* k;
+  int threads, blocks;
+  size_t smem;
+  bool operator==(const ClusterKey& o) const {
+    return dev == o.dev && k == o.k && threads == o.threads && blocks == o.blocks && smem == o.smem;
+  }
+};
+struct ClusterHash {
+  size_t operator()(const ClusterKey& o) const {
+    return std::hash<const void*>()(o.k) ^ (o.smem * 131) ^ ((size_t)o.blocks << 20) ^ ((size_t)o.dev << 40);
+  }
+};
+std::unordered_map<ClusterKey, bool, ClusterHash> g_cluster;
+}  // namespace
+
+bool cluster_fits(const void* kernel, int threads, size_t dyn_smem, int blocks) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  const ClusterKey key{dev, kernel, threads, blocks, dyn_smem};
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    auto it = g_cluster.find(key);
+    if (it != g_cluster.end()) return it->second;
+  }
+  bool ok = allow_smem(kernel, dyn_smem) == cudaSuccess;
+  if (ok && blocks > 8)
+    ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+  if (ok) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = dyn_smem;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)blocks;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    ok = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n >= 1;
+  }
+  (void)cudaGetLastError();
+  std::lock_guard<std::mutex> lk(g_mu);
+  g_cluster[key] = ok;
+  return ok;
+}
+
+namespace {
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
   static std::once_flag once;

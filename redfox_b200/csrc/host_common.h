@@ -46,6 +46,10 @@ inline cudaStream_t as_stream(void* s) { return static_cast<cudaStream_t>(s); }
 int persistent_grid(const void* kernel, int threads, size_t dyn_smem, uint64_t work_blocks);
 // Raise a kernel's dynamic shared memory limit once.
 cudaError_t allow_smem(const void* kernel, size_t bytes);
+// Whether a cluster of `blocks` blocks of the kernel can be resident on the current device
+// (looked up once per device, kernel, cluster size and shared memory); raises the kernel's
+// limits on shared memory and cluster size.
+bool cluster_fits(const void* kernel, int threads, size_t dyn_smem, int blocks);
 
 // Tensor map of `lines` 128-byte lines at `base` (a [lines][128] u8 tensor, boxes of
 // `box_lines` <= 256 lines, 128-byte swizzle) for the tile ring.  False when `base` is not 16-byte

@@ -10,6 +10,8 @@ namespace rfx {
 template <int K>
 rfx_status run_sort(SortPlan&, uint32_t);
 template <int K>
+rfx_status run_cluster(const ClusterSort&, uint32_t);
+template <int K>
 uint64_t sort_tiles_for(uint64_t, uint32_t);
 
 namespace {
@@ -38,6 +40,19 @@ rfx_status dispatch(uint32_t kb, SortPlan& s, uint32_t vb) {
     case 16: return run_sort<16>(s, vb);
     case 32: return run_sort<32>(s, vb);
     case 64: return run_sort<64>(s, vb);
+    default: return RFX_ERR_UNSUPPORTED;
+  }
+}
+
+rfx_status dispatch_cluster(uint32_t kb, const ClusterSort& c, uint32_t vb) {
+  switch (kb) {
+    case 1: return run_cluster<1>(c, vb);
+    case 2: return run_cluster<2>(c, vb);
+    case 4: return run_cluster<4>(c, vb);
+    case 8: return run_cluster<8>(c, vb);
+    case 16: return run_cluster<16>(c, vb);
+    case 32: return run_cluster<32>(c, vb);
+    case 64: return run_cluster<64>(c, vb);
     default: return RFX_ERR_UNSUPPORTED;
   }
 }
@@ -109,6 +124,17 @@ rfx_status sort_pairs_impl(void* keys, void* vals, uint64_t n, uint32_t kb, uint
   }
   SortLayout L = layout(ws, n, kb, vb, begin_bit, end_bit);
   if (!ws || ws_bytes < L.total) return RFX_ERR_WORKSPACE;
+  ClusterSort small;
+  small.keys_in = static_cast<const uint8_t*>(src_keys ? src_keys : keys);
+  small.vals_in = static_cast<const uint8_t*>(src_keys ? src_vals : vals);
+  small.keys_out = static_cast<uint8_t*>(keys);
+  small.vals_out = static_cast<uint8_t*>(vals);
+  small.n = n;
+  small.begin_bit = begin_bit;
+  small.end_bit = end_bit;
+  small.stream = stream;
+  const rfx_status one = dispatch_cluster(kb, small, vb);
+  if (one != RFX_ERR_UNSUPPORTED) return one;
   uint32_t* err = device_error_word();
   if (!err) return RFX_ERR_CUDA;
   uint8_t* cur_k = static_cast<uint8_t*>(keys);

@@ -413,6 +413,26 @@ __device__ __forceinline__ uint32_t sort_lookback(const uint32_t* status, uint32
   return prefix;
 }
 
+// Sorts the block's `count` entries in shared memory (ends with a barrier).
+static __device__ __noinline__ void order_entries(uint32_t* entries, uint32_t count, uint32_t threads) {
+  bool more = true;
+  while (more) {
+    bool moved = false;
+    for (uint32_t odd = 0; odd < 2; ++odd) {
+      for (uint32_t i = 2 * threadIdx.x + odd; i + 1 < count; i += 2 * threads) {
+        const uint32_t x = entries[i], y = entries[i + 1];
+        if (x > y) {
+          entries[i] = y;
+          entries[i + 1] = x;
+          moved = true;
+        }
+      }
+      __syncthreads();
+    }
+    more = __syncthreads_or(moved);
+  }
+}
+
 __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
@@ -580,22 +600,7 @@ sort_pass_kernel(const __grid_constant__ SortPassArgs a) {
       disorder = disorder || (i > 0 && i < tcount && entries[i - 1] > entry[j]);
     }
     if (__syncthreads_or(disorder)) {
-      bool more = true;
-      while (more) {
-        bool moved = false;
-        for (uint32_t odd = 0; odd < 2; ++odd) {
-          for (uint32_t i = 2 * t + odd; i + 1 < tcount; i += 2 * THREADS) {
-            const uint32_t x = entries[i], y = entries[i + 1];
-            if (x > y) {
-              entries[i] = y;
-              entries[i + 1] = x;
-              moved = true;
-            }
-          }
-          __syncthreads();
-        }
-        more = __syncthreads_or(moved);
-      }
+      order_entries(entries, tcount, THREADS);
 #pragma unroll
       for (int j = 0; j < IPT; ++j) entry[j] = entries[j * THREADS + t];
     }

@@ -3,6 +3,7 @@
 #pragma once
 
 #include "host_common.h"
+#include "sort_cluster.cuh"
 #include "sort_kernels.cuh"
 
 namespace rfx {
@@ -27,6 +28,16 @@ struct SortPlan {
   uint32_t* status;     // [passes][tiles][256]
   uint64_t tiles;
   uint32_t* err;
+  cudaStream_t stream;
+};
+
+struct ClusterSort {
+  const uint8_t* keys_in;
+  const uint8_t* vals_in;
+  uint8_t* keys_out;   // keys_in, or an array that does not overlap it
+  uint8_t* vals_out;
+  uint64_t n;
+  uint32_t begin_bit, end_bit;
   cudaStream_t stream;
 };
 
@@ -86,6 +97,59 @@ rfx_status run_sort_kv(SortPlan& s) {
   return RFX_OK;
 }
 
+// The one-launch sort of small inputs; RFX_ERR_UNSUPPORTED when it does not take this one
+// (nothing is launched then).  Any bit range, in place or out of place.
+template <int K, int V>
+rfx_status run_cluster_kv(const ClusterSort& c) {
+  using T = ClusterTuning<K, V>;
+  if (c.n > T::MAX) return RFX_ERR_UNSUPPORTED;
+  // as many blocks as give each about kClusterThreads elements: fewer leave SMs idle, more
+  // only add to the exchange
+  uint32_t blocks = 1;
+  while (blocks < (uint32_t)kClusterMax && blocks * kClusterThreads < c.n) blocks *= 2;
+  const uint32_t slice = ((c.n + blocks - 1) / blocks + 31) / 32 * 32;
+  auto k = sort_cluster_kernel<K, V>;
+  // the largest slice's shared memory, so that the lookups are one per cluster size
+  const size_t smem = cluster_smem<K, V>(T::SLICE);
+  if (!cluster_fits((const void*)k, kClusterThreads, smem, (int)blocks)) return RFX_ERR_UNSUPPORTED;
+  ClusterArgs a;
+  a.keys_in = c.keys_in;
+  a.vals_in = c.vals_in;
+  a.keys_out = c.keys_out;
+  a.vals_out = c.vals_out;
+  a.n = (uint32_t)c.n;
+  a.slice = slice;
+  a.inverse = (uint32_t)(((1ull << 32) + slice - 1) / slice);
+  a.begin_bit = c.begin_bit;
+  a.end_bit = c.end_bit;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(kClusterThreads);
+  cfg.dynamicSmemBytes = cluster_smem<K, V>(slice);
+  cfg.stream = c.stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = blocks;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  RFX_CUDA_TRY(cudaLaunchKernelEx(&cfg, k, a));
+  return RFX_OK;
+}
+
+template <int K>
+rfx_status run_cluster(const ClusterSort& c, uint32_t vbytes) {
+  switch (vbytes) {
+    case 0: return run_cluster_kv<K, 0>(c);
+    case 1: return run_cluster_kv<K, 1>(c);
+    case 2: return run_cluster_kv<K, 2>(c);
+    case 4: return run_cluster_kv<K, 4>(c);
+    case 8: return run_cluster_kv<K, 8>(c);
+    case 16: return run_cluster_kv<K, 16>(c);
+    default: return RFX_ERR_UNSUPPORTED;
+  }
+}
+
 template <int K>
 rfx_status run_sort(SortPlan& s, uint32_t vbytes) {
   switch (vbytes) {
@@ -113,6 +177,7 @@ uint64_t sort_tiles_for(uint64_t n, uint32_t vbytes) {
 
 #define RFX_INSTANTIATE_SORT(K)                                  \
   template rfx_status run_sort<K>(SortPlan&, uint32_t);          \
+  template rfx_status run_cluster<K>(const ClusterSort&, uint32_t); \
   template uint64_t sort_tiles_for<K>(uint64_t, uint32_t);
 
 }  // namespace rfx

@@ -263,3 +263,29 @@ def test_sort_skips_constant_digits_on_the_device(cuda, kb, vb, n, moving):
         if vb:
             assert np.array_equal(to_np(v), exp[1])
     assert R.device_status() == R.OK
+
+
+# The one-launch sort takes inputs up to 16 slices of 64 KB or 4096 elements (ClusterTuning).
+@pytest.mark.parametrize("kb,vb,most", [(1, 0, 65536), (4, 0, 65536), (8, 0, 65536), (4, 8, 65536), (16, 0, 65536),
+                                        (16, 8, 43520), (64, 16, 12800)])
+@pytest.mark.parametrize("n", [2, 31, 512, 513, 1025, 8193, "most", "above"])
+def test_sort_small_inputs_in_one_cluster(cuda, kb, vb, most, n):
+    """One block, every cluster size and its neighbours, the largest input and the first that
+    takes the general passes; constant digits first, between and last; in and out of place."""
+    n = most if n == "most" else most + 1 if n == "above" else n
+    keys = _keys(n, kb, seed=n * 5 + kb)
+    keys[:, kb // 2] &= np.uint8(0x81)
+    keys[:, kb - 1] = 7
+    vals = np.random.default_rng(n).integers(0, 256, (n, vb), dtype=np.uint8) if vb else None
+    for begin, end in ((0, kb * 8), (max(0, kb * 8 - 24), kb * 8), (max(0, kb * 8 - 13), kb * 8 - 4)):
+        a, av = _dev(keys, cuda), _dev(vals, cuda) if vb else None
+        b, bv = R.sorted_copy(a, av, begin_bit=begin, end_bit=end)
+        exp = O.sort_pairs(keys, vals, begin_bit=begin, end_bit=end) if vb else (O.sort_pairs(keys, begin_bit=begin,
+                                                                                              end_bit=end), None)
+        assert np.array_equal(to_np(a), keys)
+        R.sort_pairs(a, av, begin_bit=begin, end_bit=end)
+        for k, v in ((a, av), (b, bv)):
+            assert np.array_equal(to_np(k), exp[0]), (begin, end)
+            if vb:
+                assert np.array_equal(to_np(v), exp[1]), (begin, end)
+    assert R.device_status() == R.OK
