@@ -38,10 +38,8 @@ def gen_join_aggregate(nr=C0_R_ROWS, ns=C0_S_ROWS, key_domain=C0_KEY_DOMAIN, dev
 def join_aggregate(r, s, stream=None):
     """sort R, sort S, join on key, SUM(amount) and COUNT by key.
     Returns (keys u32, sums int64, counts u32, join_rows)."""
-    r = r.clone()
-    s = s.clone()
-    R.sort_pairs(r, begin_bit=32, end_bit=64, stream=stream)     # R on its key field
-    R.sort_pairs(s, begin_bit=64, end_bit=96, stream=stream)     # S on its key field
+    r, _ = R.sorted_copy(r, begin_bit=32, end_bit=64, stream=stream)     # R on its key field
+    s, _ = R.sorted_copy(s, begin_bit=64, end_bit=96, stream=stream)     # S on its key field
     out, total = R.join_tuples_two_step(r, 32, s, 64, 16, stream=stream)   # (key, payload, amount)
     keys, sums, counts, g = R.reduce_tuples(out, 96, 0, 64, 4, n=total, stream=stream)
     return keys, sums, counts, total
@@ -113,16 +111,14 @@ def three_relation(d1, d2, f, list_in, list_out, f_sorted=None, stream=None):
     d2s, _ = R.select_project(d2, [32, 32, 32], [(R.GE, (R.OPND_VAR, 2), (R.OPND_CONST, C2_DATE_LO), R.I32),
                                                  (R.LT, (R.OPND_VAR, 2), (R.OPND_CONST, C2_DATE_HI), R.I32)],
                               [], [32, 32], [1, 0], stream=stream)                     # (fk, pk)
-    d2s = d2s.clone()
-    R.sort_pairs(d2s, begin_bit=32, end_bit=64, stream=stream)                        # on fk
+    d2s, _ = R.sorted_copy(d2s, begin_bit=32, end_bit=64, stream=stream)               # on fk
     j1, _ = R.join_tuples_two_step(d1s, 8, d2s, 32, 16, stream=stream)                 # (pk1, seg, pk2)
-    keys = R.project(j1, [32, 8, 32], [32], [2], stream=stream).view(torch.int32).view(-1).clone()
-    R.sort_pairs(keys, stream=stream)
+    keys = R.project(j1, [32, 8, 32], [32], [2], stream=stream).view(torch.int32).view(-1)
+    keys, _ = R.sorted_copy(keys, stream=stream)
     keys = R.set_op(R.SET_INTERSECTION, keys, list_in, stream=stream)
     keys = R.set_op(R.SET_DIFFERENCE, keys, list_out, stream=stream)
     if f_sorted is None:
-        f_sorted = f.clone()
-        R.sort_pairs(f_sorted, begin_bit=64, end_bit=96, stream=stream)               # on fk
+        f_sorted, _ = R.sorted_copy(f, begin_bit=64, end_bit=96, stream=stream)       # on fk
     keys4 = keys.view(torch.uint8).view(-1, 4)
     j2, total = R.join_tuples_two_step(keys4, 0, f_sorted, 64, 16, stream=stream)     # (pk2, amount)
     gk, gs, gc, _ = R.reduce_tuples(j2, 64, 0, 64, 4, n=total, stream=stream)
