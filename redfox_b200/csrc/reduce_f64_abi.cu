@@ -2,18 +2,23 @@
 // (thrust::reduce_by_key with plus<double>), min_32_double (minimum<double>) and the
 // scalar total_double / max_double / count of Reduce.cu:742-1536.
 //
-// Sums are exact, then rounded once (round to nearest, ties to even): every double is a
-// 53-bit integer times a power of two, so a run's sum is accumulated as a two's-complement
-// integer in units of 2^L over W 64-bit limbs (add with carry).  Integer addition is
-// associative, so the result does not depend on how the work is split -- unlike a
-// floating-point tree, whose rounding follows its shape.  The fast window is W = 3 limbs
-// with L set from the largest exponent in the input (a pre-pass): exact for every value
-// within 2^107 of the largest, with room for 2^30 terms.  A value below that window with
-// bits that would be lost raises a flag, and a second pass with W = 34 limbs and
-// L = -1074, which covers every finite double, runs -- its kernels are always enqueued and
-// return at once unless the flag is set, so no host round trip is needed.  Specials
-// follow IEEE addition: NaN if any NaN or both infinities, else the infinity, and an
-// exact zero is -0 only when every term is -0.
+// Sums are exact, then rounded once (round to nearest, ties to even), in up to three passes.
+//   * The first keeps a run's sum as an unevaluated pair of doubles hi + lo.  Every addition
+//     is an error-free transformation (Knuth's TwoSum, both parts): the error of the high
+//     addition goes to the low part, and an error of the low addition raises a flag.  While
+//     the flag stays down hi + lo is the exact sum whatever the order of the additions, and
+//     one rounding of hi + lo finishes it.  This holds for values whose bits span about 100
+//     binary places, such as amounts of money.
+//   * If the flag went up (a wider span, an overflow, an infinity or a NaN), a second pass
+//     works in integers: every double is a 53-bit integer times a power of two, so a run's
+//     sum is accumulated as a two's-complement integer in units of 2^L over W 64-bit limbs
+//     (add with carry).  W = 3 limbs with L set from the largest exponent in the input: exact
+//     for every value within 2^107 of the largest, with room for 2^30 terms.
+//   * A value below that window with bits that would be lost raises a flag too, and a third
+//     pass with W = 34 limbs and L = -1074, which covers every finite double, runs.
+// The kernels of the later passes are always enqueued and return at once unless their flag is
+// set, so no host round trip is needed.  Specials follow IEEE addition: NaN if any NaN or both
+// infinities, else the infinity, and an exact zero is -0 only when every term is -0.
 //
 // The minimum follows the reference's fold acc = (acc < v ? acc : v) exactly: a later
 // element replaces an equal one (so -0 / +0 ties go to the later), a NaN sets the
@@ -21,12 +26,12 @@
 // combination of run summaries, so the parallel result equals the sequential one bit for
 // bit.
 //
-// Structure: units of 4096 elements, one warp per unit.  A pre-pass counts each unit's run
-// heads (taking the exponent maximum for sums) and one block scans the counts into each
-// unit's first run index; the main pass folds a unit in registers and warp shuffles,
-// writes every run that starts and ends inside it at its final index, and leaves the
-// partial before its first head and the partial from its last head for the fix-up, a
-// segmented scan over units that closes the runs crossing units.
+// Structure: units of up to 4096 elements, one warp per unit.  A pre-pass counts each unit's
+// run heads, and its last block scans the counts into each unit's first run index; the main
+// pass folds a unit in registers and warp shuffles, writes every run that starts and ends
+// inside it at its final index, and leaves the partial before its first head and the partial
+// from its last head for the fix-up, which closes the runs crossing units.
+//
 #include <cstring>
 
 #include "host_common.h"
@@ -35,7 +40,6 @@
 namespace rfx {
 namespace {
 
-constexpr int kFixThreads = 256;
 constexpr int kNarrowLimbs = 3;   // 192 bits: every value within 2^107 of the largest
 constexpr int kWideLimbs = 34;    // 2176 bits: every finite double
 constexpr int kWideL = -1074;
@@ -48,6 +52,7 @@ enum : uint32_t { kSumNaN = 1, kSumPosInf = 2, kSumNegInf = 4, kSumNotNegZero = 
 // choice of L, so the result is exact and independent of the order of the additions.
 template <int W>
 struct SumOp {
+  static constexpr int BLOCKS = W == 3 ? 2 : 1;   // of 256 threads per SM: the limbs live in registers
   struct P {
     unsigned long long l[W];
     uint32_t flags;
@@ -91,7 +96,7 @@ struct SumOp {
       }
     }
   }
-  __device__ __forceinline__ static void add(P& p, double x, int L, uint32_t* inexact) {
+  __device__ __forceinline__ static void add(P& p, double x, int L, uint32_t* inexact, bool&) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(x);
     const uint32_t eb = (uint32_t)(b >> 52) & 0x7ffu;
     const unsigned long long frac = b & ((1ull << 52) - 1);
@@ -119,7 +124,7 @@ struct SumOp {
     const unsigned long long hi = o ? m >> (64 - o) : 0ull;
     accumulate(p.l, q, lo, hi, neg);
   }
-  __device__ __forceinline__ static P combine(const P& a, const P& b) {
+  __device__ __forceinline__ static P combine(const P& a, const P& b, bool&) {
     P r;
     if constexpr (W == 3) {
       r.l[0] = a.l[0];
@@ -206,15 +211,51 @@ struct SumOp {
   }
 };
 
+// ------------------------------------------------------------------ exact sum in two doubles
+// The sum is hi + lo exactly as long as no flag (`bad`) went up.
+struct PairOp {
+  static constexpr int BLOCKS = 4;
+  struct P {
+    double hi, lo;
+  };
+  __device__ __forceinline__ static P identity() { return P{-0.0, 0.0}; }   // -0 + x is x for every x
+  // a + b = s + e exactly (Knuth's TwoSum); e is NaN after an overflow or a special.
+  __device__ __forceinline__ static double two_sum(double a, double b, double& e) {
+    const double s = __dadd_rn(a, b);
+    const double bb = __dadd_rn(s, -a);
+    e = __dadd_rn(__dadd_rn(a, -__dadd_rn(s, -bb)), __dadd_rn(b, -bb));
+    return s;
+  }
+  __device__ __forceinline__ static void add(P& p, double x, int, uint32_t*, bool& bad) {
+    double e, e2;
+    p.hi = two_sum(p.hi, x, e);
+    p.lo = two_sum(p.lo, e, e2);
+    bad = bad || !(e2 == 0.0);   // a NaN is not zero
+  }
+  __device__ __forceinline__ static P combine(const P& a, const P& b, bool& bad) {
+    double e, e2, e3, r;
+    const double s = two_sum(a.hi, b.hi, e);
+    const double l = two_sum(a.lo, b.lo, e2);
+    const double t = two_sum(l, e, e3);
+    bad = bad || !(e2 == 0.0) || !(e3 == 0.0);
+    const double h = two_sum(s, t, r);   // keeps the low part below the high one's last place
+    return t == 0.0 ? P{s, 0.0} : P{h, r};   // (s + 0 would lose the sign of a zero)
+  }
+  __device__ __forceinline__ static unsigned long long finalize(const P& p, int) {
+    return (unsigned long long)__double_as_longlong(p.lo == 0.0 ? p.hi : __dadd_rn(p.hi, p.lo));
+  }
+};
+
 // ------------------------------------------------------------------ minimum (the fold)
 struct MinOp {
+  static constexpr int BLOCKS = 4;
   struct P {
     unsigned long long v;  // bits of the fold value (a NaN while pending)
     uint32_t any;          // an element after the last NaN was folded
     uint32_t nan;          // a NaN occurs in the summarised range
   };
   __device__ __forceinline__ static P identity() { return P{0ull, 0u, 0u}; }
-  __device__ __forceinline__ static void add(P& p, double x, int, uint32_t*) {
+  __device__ __forceinline__ static void add(P& p, double x, int, uint32_t*, bool&) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(x);
     if (x != x) {
       p = P{b, 0u, 1u};
@@ -227,7 +268,7 @@ struct MinOp {
     }
   }
   // a is the earlier range, b the later one.
-  __device__ __forceinline__ static P combine(const P& a, const P& b) {
+  __device__ __forceinline__ static P combine(const P& a, const P& b, bool&) {
     if (b.nan) return b;
     if (!b.any) return a;
     if (!a.any) return P{b.v, 1u, a.nan};
@@ -236,6 +277,12 @@ struct MinOp {
   }
   __device__ static unsigned long long finalize(const P& p, int) { return p.v; }
 };
+
+__device__ __forceinline__ uint32_t ld_relaxed_u32(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
 
 // ------------------------------------------------------------------ keys
 struct Key {
@@ -265,25 +312,7 @@ __device__ __forceinline__ void store_key(uint8_t* out, uint64_t r, const Key& k
   if constexpr (KB == 16) reinterpret_cast<ulonglong2*>(out)[r] = make_ulonglong2(k.lo, k.hi);
 }
 
-// ------------------------------------------------------------------ segmented scan
-template <typename P>
-struct Seg {
-  P v;
-  uint32_t f;  // a head (run start) lies in the summarised range
-  uint32_t pad;
-};
-
-template <class Op>
-__device__ __forceinline__ Seg<typename Op::P> seg_combine(const Seg<typename Op::P>& a,
-                                                           const Seg<typename Op::P>& b) {
-  if (b.f) return b;
-  Seg<typename Op::P> r;
-  r.v = Op::combine(a.v, b.v);
-  r.f = a.f;
-  r.pad = 0;
-  return r;
-}
-
+// ------------------------------------------------------------------ shuffles
 template <typename T>
 __device__ __forceinline__ T shfl_up_any(const T& x, int delta) {
   constexpr int W = (int)((sizeof(T) + 3) / 4);
@@ -291,6 +320,18 @@ __device__ __forceinline__ T shfl_up_any(const T& x, int delta) {
   memcpy(w, &x, sizeof(T));
 #pragma unroll
   for (int i = 0; i < W; ++i) w[i] = __shfl_up_sync(0xffffffffu, w[i], delta);
+  T r;
+  memcpy(&r, w, sizeof(T));
+  return r;
+}
+
+template <typename T>
+__device__ __forceinline__ T shfl_down_any(const T& x, int delta) {
+  constexpr int W = (int)((sizeof(T) + 3) / 4);
+  uint32_t w[W];
+  memcpy(w, &x, sizeof(T));
+#pragma unroll
+  for (int i = 0; i < W; ++i) w[i] = __shfl_down_sync(0xffffffffu, w[i], delta);
   T r;
   memcpy(&r, w, sizeof(T));
   return r;
@@ -308,276 +349,223 @@ __device__ __forceinline__ T shfl_any(const T& x, int src) {
   return r;
 }
 
-// Exclusive segmented scan over the NT threads of a block (thread order); also returns the
-// block's inclusive total.  `warp_tot` holds NT / 32 entries.
-template <class Op, int NT>
-__device__ Seg<typename Op::P> block_seg_scan(const Seg<typename Op::P>& x, Seg<typename Op::P>* warp_tot,
-                                              Seg<typename Op::P>& total) {
-  using S = Seg<typename Op::P>;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  S inc = x;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const S y = shfl_up_any(inc, o);
-    if (lane >= o) inc = seg_combine<Op>(y, inc);
-  }
-  S exc = shfl_up_any(inc, 1);
-  if (lane == 31) warp_tot[warp] = inc;
-  __syncthreads();
-  S pre;
-  pre.v = Op::identity();
-  pre.f = 0;
-  pre.pad = 0;
-  for (int w = 0; w < warp; ++w) pre = seg_combine<Op>(pre, warp_tot[w]);
-  if (lane == 0) {
-    exc = pre;
-  } else {
-    exc = seg_combine<Op>(pre, exc);
-  }
-  total = pre;
-  for (int w = warp; w < NT / 32; ++w) total = seg_combine<Op>(total, warp_tot[w]);
-  __syncthreads();
-  return exc;
-}
-
 // ------------------------------------------------------------------ kernels
 struct F64Args {
   const uint8_t* keys;
   const double* vals;
   uint64_t n;
+  uint32_t unit;        // elements per unit, a multiple of kF64Step
   const unsigned long long* emit;  // if set, out key of a run = emit[head] (8 bytes)
   uint8_t* out_keys;
   double* out_vals;
   uint64_t* d_groups;
-  uint64_t* status;     // look-back words, one per tile
-  uint32_t* counter;    // tile counter
-  uint32_t* tile_heads;
-  uint32_t* tile_base;
-  void* tile_first;     // Op::P per tile
-  void* tile_last;
-  void* exc;            // Seg<P> per tile (fix-up)
-  void* chunk_agg;      // Seg<P> per fix-up chunk
-  const int* d_emax;    // max biased exponent (sums with the narrow window)
-  int fixed_L;          // used when d_emax is null
-  uint32_t* inexact;
-  const uint32_t* gate;   // if set, the kernels do nothing unless *gate != 0
+  uint32_t* done;       // blocks of the count that have finished
+  uint32_t* heads;      // run heads per unit
+  uint32_t* base;       // index of the unit's first run (heads before it)
+  void* first;          // Op::P per unit: before its first head (the whole unit if it has none)
+  void* last;           // Op::P per unit: from its last head
+  int* emax;            // max biased exponent of the finite values (the 3-limb pass's window)
+  int fixed_L;          // used when emax is null
+  uint32_t* inexact;    // raised when the pass could not be exact
+  const uint32_t* gate; // if set, the kernels do nothing unless *gate != 0
   uint32_t* err;
 };
 
 __device__ __forceinline__ bool gated_off(const F64Args& a) { return a.gate && *a.gate == 0u; }
 
 __device__ __forceinline__ int window_L(const F64Args& a) {
-  if (!a.d_emax) return a.fixed_L;
-  const int e = *a.d_emax;
+  if (!a.emax) return a.fixed_L;
+  const int e = *a.emax;
   return (e > 1 ? e : 1) - 1182;
 }
 
-// Fix-up, step 1: per chunk of kFixThreads tiles, the exclusive segmented scan of the
-// tile summaries (a tile with a head contributes its last partial, else its whole sum).
-template <class Op>
-__global__ void __launch_bounds__(kFixThreads) f64_fix_scan(F64Args a, uint64_t tiles) {
-  if (gated_off(a)) return;
-  using P = typename Op::P;
-  using S = Seg<P>;
-  __shared__ S s_warp[kFixThreads / 32];
-  const uint64_t u = (uint64_t)blockIdx.x * kFixThreads + threadIdx.x;
-  S x;
-  x.pad = 0;
-  if (u < tiles) {
-    x.f = a.tile_heads[u] > 0;
-    x.v = x.f ? reinterpret_cast<const P*>(a.tile_last)[u] : reinterpret_cast<const P*>(a.tile_first)[u];
-  } else {
-    x.f = 0;
-    x.v = Op::identity();
-  }
-  S total;
-  const S e = block_seg_scan<Op, kFixThreads>(x, s_warp, total);
-  if (u < tiles) reinterpret_cast<S*>(a.exc)[u] = e;
-  if (threadIdx.x == 0) reinterpret_cast<S*>(a.chunk_agg)[blockIdx.x] = total;
-}
-
-// Step 2: exclusive segmented scan over the chunk aggregates (one block, in order).
-template <class Op>
-__global__ void __launch_bounds__(kFixThreads) f64_fix_chunks(F64Args a, uint64_t chunks) {
-  if (gated_off(a)) return;
-  using S = Seg<typename Op::P>;
-  __shared__ S s_warp[kFixThreads / 32];
-  __shared__ S s_carry;
-  if (threadIdx.x == 0) {
-    s_carry.v = Op::identity();
-    s_carry.f = 0;
-    s_carry.pad = 0;
-  }
-  __syncthreads();
-  S* agg = reinterpret_cast<S*>(a.chunk_agg);
-  for (uint64_t base = 0; base < chunks; base += kFixThreads) {
-    const uint64_t c = base + threadIdx.x;
-    S x;
-    if (c < chunks) {
-      x = agg[c];
-    } else {
-      x.v = Op::identity();
-      x.f = 0;
-      x.pad = 0;
-    }
-    S total;
-    const S e = block_seg_scan<Op, kFixThreads>(x, s_warp, total);
-    const S carry = s_carry;
-    __syncthreads();
-    if (c < chunks) agg[c] = seg_combine<Op>(carry, e);  // now the chunk's exclusive prefix
-    if (threadIdx.x == 0) s_carry = seg_combine<Op>(carry, total);
-    __syncthreads();
-  }
-}
-
-// Step 3: the runs that cross tile boundaries.  Tile u with a head closes the run of the
-// previous head (the last head of an earlier tile); the last tile also closes the last run.
-template <class Op>
-__global__ void __launch_bounds__(kFixThreads) f64_fix_apply(F64Args a, uint64_t tiles) {
-  if (gated_off(a)) return;
-  using P = typename Op::P;
-  using S = Seg<P>;
-  const uint64_t u = (uint64_t)blockIdx.x * kFixThreads + threadIdx.x;
-  if (u >= tiles) return;
-  const int L = window_L(a);
-  const S pre = reinterpret_cast<const S*>(a.chunk_agg)[blockIdx.x];
-  const S x = seg_combine<Op>(pre, reinterpret_cast<const S*>(a.exc)[u]);
-  const bool has_head = a.tile_heads[u] > 0;
-  if (has_head && x.f) {
-    const P y = Op::combine(x.v, reinterpret_cast<const P*>(a.tile_first)[u]);
-    a.out_vals[a.tile_base[u] - 1] = __longlong_as_double((long long)Op::finalize(y, L));
-  }
-  if (u == tiles - 1) {
-    S self;
-    self.f = has_head;
-    self.v = has_head ? reinterpret_cast<const P*>(a.tile_last)[u] : reinterpret_cast<const P*>(a.tile_first)[u];
-    self.pad = 0;
-    const S y = seg_combine<Op>(x, self);
-    a.out_vals[a.tile_base[u] + a.tile_heads[u] - 1] = __longlong_as_double((long long)Op::finalize(y.v, L));
-  }
-}
-
-// ------------------------------------------------------------------ warp units
-// The default path: units of kF64UnitItems elements, one warp per unit.  A pre-pass counts
-// every unit's run heads (and takes the exponent maximum for sums); one block scans the
-// counts into each unit's first run index.  The main pass then needs nothing from other
-// units: a warp folds its unit in 256-element steps (8 per lane) with shuffles only,
-// writes every run that starts and ends inside the unit at its final index, and leaves the
-// partial before the unit's first head and the partial from its last head for the fix-up
-// above, which treats units as tiles.
-constexpr int kF64UnitItems = 4096;
 constexpr int kF64WarpIPT = 8;
+constexpr int kF64Step = 32 * kF64WarpIPT;   // elements a warp folds at a time
+constexpr int kF64UnitMost = 4096;
 
+// Eight consecutive keys from element `first` (a multiple of 8) of a 16-byte aligned array.
 template <int KB>
-__global__ void __launch_bounds__(256) f64_unit_count(F64Args a, uint64_t units, int* emax) {
-  if (gated_off(a)) return;
-  const uint32_t lane = threadIdx.x & 31;
-  const uint64_t gw = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  int m = 1;
-  for (uint64_t u = gw; u < units; u += nw) {
-    const uint64_t e0 = u * kF64UnitItems, e1 = min(e0 + (uint64_t)kF64UnitItems, a.n);
+__device__ __forceinline__ void load_keys8(const uint8_t* keys, uint64_t first, Key (&k)[8]) {
+  const uint8_t* p = keys + first * KB;
+  if constexpr (KB == 1) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) k[j] = Key{((j < 4 ? v.x : v.y) >> (8 * (j & 3))) & 0xffu, 0ull};
+  } else if constexpr (KB == 2) {
+    const uint4 v = *reinterpret_cast<const uint4*>(p);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) k[j] = Key{(w[j >> 1] >> (16 * (j & 1))) & 0xffffu, 0ull};
+  } else if constexpr (KB == 4) {
+    const uint4 a = reinterpret_cast<const uint4*>(p)[0], b = reinterpret_cast<const uint4*>(p)[1];
+    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) k[j] = Key{w[j], 0ull};
+  } else if constexpr (KB == 8) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const ulonglong2 v = reinterpret_cast<const ulonglong2*>(p)[j];
+      k[2 * j] = Key{v.x, 0ull};
+      k[2 * j + 1] = Key{v.y, 0ull};
+    }
+  } else if constexpr (KB == 16) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const ulonglong2 v = reinterpret_cast<const ulonglong2*>(p)[j];
+      k[j] = Key{v.x, v.y};
+    }
+  }
+}
+
+// Keys first .. first + 7 of the elements before `end`; vec: the array is 16-byte aligned.
+template <int KB>
+__device__ __forceinline__ void load_keys(const uint8_t* keys, uint64_t first, uint64_t end, bool vec, Key (&k)[8]) {
+  if constexpr (KB == 0) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) k[j] = Key{0ull, 0ull};
+  } else if (vec && first + 8 <= end) {
+    load_keys8<KB>(keys, first, k);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) k[j] = first + j < end ? load_key<KB>(keys, first + j) : Key{0ull, 0ull};
+  }
+}
+
+// The heads among a lane's keys (bit j: element first + j starts a run).
+template <int KB>
+__device__ __forceinline__ uint32_t head_bits(const F64Args& a, const Key (&k)[8], uint64_t first, uint64_t end) {
+  uint32_t hm = first == 0 && end > 0 ? 1u : 0u;
+  if constexpr (KB > 0) {
+    const uint32_t lane = threadIdx.x & 31;
+    Key pk;
+    pk.lo = __shfl_up_sync(0xffffffffu, k[7].lo, 1);
+    pk.hi = KB == 16 ? __shfl_up_sync(0xffffffffu, k[7].hi, 1) : 0ull;
+    if (lane == 0 && first > 0 && first < end) pk = load_key<KB>(a.keys, first - 1);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const Key q = j ? k[j - 1] : pk;
+      const bool h = first + j > 0 && first + j < end && (k[j].lo != q.lo || k[j].hi != q.hi);
+      hm |= (uint32_t)h << j;
+    }
+  }
+  return hm;
+}
+
+// Run heads per unit, one warp per unit; the last block to finish turns the counts into each
+// unit's first run index and writes the number of runs.
+template <int KB>
+__global__ void __launch_bounds__(256) f64_unit_count(F64Args a, uint64_t units) {
+  __shared__ uint64_t s_warp[8];
+  __shared__ bool s_last;
+  const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const bool vec = (reinterpret_cast<uintptr_t>(a.keys) & 15u) == 0;
+  const uint64_t nw = (uint64_t)gridDim.x * 8;
+  for (uint64_t u = (uint64_t)blockIdx.x * 8 + warp; u < units; u += nw) {
+    const uint64_t e0 = u * a.unit, e1 = min(e0 + (uint64_t)a.unit, a.n);
     uint32_t c = 0;
-    for (uint64_t e = e0 + lane; e < e1; e += 32) {
-      bool h = e == 0;
-      if constexpr (KB > 0) {
-        if (!h) {
-          const Key k = load_key<KB>(a.keys, e), pk = load_key<KB>(a.keys, e - 1);
-          h = k.lo != pk.lo || k.hi != pk.hi;
-        }
-      }
-      c += h;
-      if (emax) {
-        const int eb = (int)(((unsigned long long)__double_as_longlong(a.vals[e]) >> 52) & 0x7ffu);
-        if (eb != 0x7ff && eb > m) m = eb;
-      }
+#pragma unroll 4
+    for (uint64_t tb = e0; tb < e1; tb += kF64Step) {
+      const uint64_t first = tb + 8ull * lane;
+      Key k[8];
+      load_keys<KB>(a.keys, first, e1, vec, k);
+      c += (uint32_t)__popc(head_bits<KB>(a, k, first, e1));
     }
     c = __reduce_add_sync(0xffffffffu, c);
-    if (lane == 0) a.tile_heads[u] = c;
+    if (lane == 0) a.heads[u] = c;
   }
-  if (emax) {
-    m = __reduce_max_sync(0xffffffffu, m);
-    if (lane == 0) atomicMax(emax, m);
-  }
-}
-
-// Exclusive scan of the unit head counts (one block, in order) and the number of runs.
-__global__ void __launch_bounds__(1024) f64_unit_scan(F64Args a, uint64_t units) {
-  if (gated_off(a)) return;
-  __shared__ uint32_t s_warp[32];
-  __shared__ uint64_t s_carry;
-  const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  if (t == 0) s_carry = 0;
+  __threadfence();
   __syncthreads();
-  for (uint64_t b = 0; b < units; b += 1024) {
-    const uint64_t u = b + t;
-    const uint32_t x = u < units ? a.tile_heads[u] : 0u;
-    uint32_t inc = x;
+  if (t == 0) s_last = atomicAdd(a.done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  // consecutive counts per thread, 8 at a time
+  uint64_t carry = 0;
+  for (uint64_t b = 0; b < units; b += 8 * 256) {
+    uint32_t c[8], sum = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint64_t u = b + 8ull * t + j;
+      c[j] = u < units ? ld_relaxed_u32(a.heads + u) : 0u;
+      sum += c[j];
+    }
+    uint64_t inc = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+      const uint64_t y = __shfl_up_sync(0xffffffffu, inc, o);
       if (lane >= (uint32_t)o) inc += y;
     }
     if (lane == 31) s_warp[warp] = inc;
     __syncthreads();
-    uint32_t wpre = 0, tot = 0;
-    for (uint32_t w = 0; w < 32; ++w) {
-      if (w < warp) wpre += s_warp[w];
-      tot += s_warp[w];
+    uint64_t run = carry + inc - sum;
+#pragma unroll
+    for (uint32_t w = 0; w < 8; ++w) {
+      run += w < warp ? s_warp[w] : 0ull;
+      carry += s_warp[w];
     }
-    const uint64_t carry = s_carry;
-    if (u < units) a.tile_base[u] = (uint32_t)(carry + wpre + inc - x);
-    __syncthreads();
-    if (t == 0) s_carry = carry + tot;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint64_t u = b + 8ull * t + j;
+      if (u < units) a.base[u] = (uint32_t)run;
+      run += c[j];
+    }
     __syncthreads();
   }
-  if (t == 0) *a.d_groups = s_carry;
+  if (t == 0) *a.d_groups = carry;
 }
 
+// The largest biased exponent of the finite values (the 3-limb pass's window).
+__global__ void __launch_bounds__(256) f64_emax(F64Args a) {
+  if (gated_off(a)) return;
+  int m = 1;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += (uint64_t)gridDim.x * blockDim.x) {
+    const int eb = (int)(((unsigned long long)__double_as_longlong(a.vals[i]) >> 52) & 0x7ffu);
+    if (eb != 0x7ff && eb > m) m = eb;
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) atomicMax(a.emax, m);
+}
+
+// The main pass: a warp folds its unit 256 elements at a time, 8 consecutive ones per lane
+// (16-byte loads).  A lane folds its elements, writing the runs that start and end among
+// them; a segmented warp scan gives every lane what is open before it.  Bound by the latency
+// of a step's chain (loads, fold, scan), so by the warps resident: 19.3M elements, 256K runs,
+// SUM with 32 warps per SM (64 registers) 87 us, with 24 warps 105, with 16 warps and the next
+// step's loads in flight 106, the 3-limb integers 174; MIN 73 / 98 / 90, before 100.
 template <int KB, class Op>
-__global__ void __launch_bounds__(256) f64_unit_kernel(F64Args a, uint64_t units) {
+__global__ void __launch_bounds__(256, Op::BLOCKS) f64_unit_kernel(F64Args a, uint64_t units) {
   if (gated_off(a)) return;
   using P = typename Op::P;
-  using S = Seg<P>;
   constexpr int V = kF64WarpIPT;
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t gw = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   const int L = window_L(a);
+  const bool vk = (reinterpret_cast<uintptr_t>(a.keys) & 15u) == 0;
+  const bool vv = (reinterpret_cast<uintptr_t>(a.vals) & 15u) == 0;
+  bool bad = false;
   for (uint64_t u = gw; u < units; u += nw) {
-    const uint64_t e0 = u * kF64UnitItems, e1 = min(e0 + (uint64_t)kF64UnitItems, a.n);
-    const uint64_t ubase = a.tile_base[u];
-    S carry;
-    carry.v = Op::identity();
-    carry.f = 0;
-    carry.pad = 0;
-    uint64_t heads_so_far = 0;
-    for (uint64_t tb = e0; tb < e1; tb += 32 * V) {
+    const uint64_t e0 = u * a.unit, e1 = min(e0 + (uint64_t)a.unit, a.n);
+    uint64_t run_base = a.base[u];   // index of the next head's run
+    P carry = Op::identity();
+    bool carry_head = false;
+    for (uint64_t tb = e0; tb < e1; tb += kF64Step) {
       const uint64_t first = tb + (uint64_t)lane * V;
       Key keys[V];
       double vals[V];
-      uint32_t hm = 0;
+      load_keys<KB>(a.keys, first, e1, vk, keys);
+      if (vv && first + V <= e1) {
 #pragma unroll
-      for (int j = 0; j < V; ++j) {
-        keys[j] = Key{0ull, 0ull};
-        vals[j] = 0.0;
-        if (first + j < e1) {
-          keys[j] = load_key<KB>(a.keys, first + j);
-          vals[j] = a.vals[first + j];
+        for (int j = 0; j < V / 2; ++j) {
+          const double2 v = reinterpret_cast<const double2*>(a.vals + first)[j];
+          vals[2 * j] = v.x;
+          vals[2 * j + 1] = v.y;
         }
-      }
-      Key pk;
-      pk.lo = __shfl_sync(0xffffffffu, keys[V - 1].lo, lane ? lane - 1 : 0);
-      pk.hi = __shfl_sync(0xffffffffu, keys[V - 1].hi, lane ? lane - 1 : 0);
-      if (lane == 0 && first > 0 && first < e1) pk = load_key<KB>(a.keys, first - 1);
+      } else {
 #pragma unroll
-      for (int j = 0; j < V; ++j) {
-        if (first + j < e1) {
-          const Key q = j ? keys[j - 1] : pk;
-          const bool h = first + j == 0 || (KB > 0 && (keys[j].lo != q.lo || keys[j].hi != q.hi));
-          hm |= (uint32_t)h << j;
-        }
+        for (int j = 0; j < V; ++j) vals[j] = first + j < e1 ? a.vals[first + j] : 0.0;
       }
+      const uint32_t hm = head_bits<KB>(a, keys, first, e1);
       // run index of this lane's first head
       const uint32_t cnt = (uint32_t)__popc(hm);
       uint32_t inc = cnt;
@@ -586,67 +574,105 @@ __global__ void __launch_bounds__(256) f64_unit_kernel(F64Args a, uint64_t units
         const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
         if (lane >= (uint32_t)o) inc += y;
       }
-      const uint32_t ttot = __shfl_sync(0xffffffffu, inc, 31);
-      const uint64_t run_base = ubase + heads_so_far + (inc - cnt);
+      const uint64_t lane_run = run_base + inc - cnt;
       // keys at heads; runs that end inside this lane
       P cur = Op::identity(), pfirst = Op::identity();
-      bool seen = false;
-      uint32_t r = 0;
+      uint64_t r = lane_run;
 #pragma unroll
       for (int j = 0; j < V; ++j) {
         if (first + j < e1) {
           if ((hm >> j) & 1u) {
             if (a.emit)
-              reinterpret_cast<unsigned long long*>(a.out_keys)[run_base + r] = a.emit[first + j];
+              reinterpret_cast<unsigned long long*>(a.out_keys)[r] = a.emit[first + j];
             else
-              store_key<KB>(a.out_keys, run_base + r, keys[j]);
-            if (seen)
-              a.out_vals[run_base + r - 1] = __longlong_as_double((long long)Op::finalize(cur, L));
+              store_key<KB>(a.out_keys, r, keys[j]);
+            if (r != lane_run)
+              a.out_vals[r - 1] = __longlong_as_double((long long)Op::finalize(cur, L));
             else
               pfirst = cur;
             cur = Op::identity();
-            seen = true;
             ++r;
           }
-          Op::add(cur, vals[j], L, a.inexact);
+          Op::add(cur, vals[j], L, a.inexact, bad);
         }
       }
+      const bool seen = cnt != 0;
       if (!seen) pfirst = cur;
-      // everything before this lane in the unit, then the run that ends before its first head
-      S x;
-      x.v = seen ? cur : pfirst;
-      x.f = seen;
-      x.pad = 0;
-      S incl = x;
+      // what is open before each lane: inclusive scan of the lanes' last partials, from the
+      // nearest lane with a head on
+      const uint32_t seen_mask = __ballot_sync(0xffffffffu, seen);
+      const uint32_t upto = seen_mask & (0xffffffffu >> (31 - lane));
+      const uint32_t start = upto ? 31u - __clz(upto) : 0u;
+      P incl = cur;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const S y = shfl_up_any(incl, o);
-        if (lane >= (uint32_t)o) incl = seg_combine<Op>(y, incl);
+        const P y = shfl_up_any(incl, o);
+        if (lane >= start + o) incl = Op::combine(y, incl, bad);
       }
-      S ex = shfl_up_any(incl, 1);
-      if (lane == 0) {
-        ex.v = Op::identity();
-        ex.f = 0;
-        ex.pad = 0;
-      }
-      const S X = seg_combine<Op>(carry, ex);
+      P X = shfl_up_any(incl, 1);
+      if (lane == 0) X = Op::identity();
+      const bool before = (seen_mask & ((1u << lane) - 1)) != 0;
+      const P all = shfl_any(incl, 31);
       if (seen) {
-        const P y = Op::combine(X.v, pfirst);
-        if (X.f)
-          a.out_vals[run_base - 1] = __longlong_as_double((long long)Op::finalize(y, L));
+        // the run that ends before this lane's first head
+        const P y = Op::combine(before ? X : Op::combine(carry, X, bad), pfirst, bad);
+        if (before || carry_head)
+          a.out_vals[lane_run - 1] = __longlong_as_double((long long)Op::finalize(y, L));
         else
-          reinterpret_cast<P*>(a.tile_first)[u] = y;   // the run began before this unit
+          reinterpret_cast<P*>(a.first)[u] = y;   // the run began before this unit
       }
-      const S tt = shfl_any(incl, 31);
-      carry = seg_combine<Op>(carry, tt);
-      heads_so_far += ttot;
+      carry = seen_mask ? all : Op::combine(carry, all, bad);
+      carry_head = carry_head || seen_mask != 0;
+      run_base += __shfl_sync(0xffffffffu, inc, 31);
     }
-    if (lane == 0) {
-      if (carry.f)
-        reinterpret_cast<P*>(a.tile_last)[u] = carry.v;
-      else
-        reinterpret_cast<P*>(a.tile_first)[u] = carry.v;
+    if (lane == 0) reinterpret_cast<P*>(carry_head ? a.last : a.first)[u] = carry;
+  }
+  if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.inexact, 1u);
+}
+
+// The runs that cross units, one warp per unit: a unit with a head closes the run of the last
+// head before it, the last unit also the last run.  The warp walks back over the units
+// without a head, 32 at a time; every unit is walked over by one warp only.
+template <class Op>
+__global__ void __launch_bounds__(256) f64_fix(F64Args a, uint64_t units) {
+  if (gated_off(a)) return;
+  using P = typename Op::P;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t u = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (u >= units) return;
+  const int L = window_L(a);
+  const bool head = a.heads[u] > 0, last = u == units - 1;
+  if (!head && !last) return;
+  const P* first_of = reinterpret_cast<const P*>(a.first);
+  const P* last_of = reinterpret_cast<const P*>(a.last);
+  bool bad = false;
+  P acc = Op::identity();
+  int64_t pos = (int64_t)u - 1;
+  while (pos >= 0) {
+    const int64_t v = pos - lane;
+    const bool h = v >= 0 && a.heads[v] > 0;
+    const uint32_t m = __ballot_sync(0xffffffffu, h);
+    const uint32_t stop = m ? __ffs(m) - 1 : 31u;   // the nearest unit with a head
+    P x = v >= 0 && lane <= stop ? (h ? last_of[v] : first_of[v]) : Op::identity();
+    // in order: a higher lane holds an earlier unit
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const P y = shfl_down_any(x, o);
+      if (lane + o < 32) x = Op::combine(y, x, bad);
     }
+    acc = Op::combine(shfl_any(x, 0), acc, bad);
+    if (m) break;
+    pos -= 32;
+  }
+  if (lane == 0) {
+    const uint64_t base = a.base[u];
+    if (u > 0) {
+      const P y = Op::combine(acc, first_of[u], bad);
+      a.out_vals[base - 1] = __longlong_as_double((long long)Op::finalize(y, L));
+    }
+    if (last && head)
+      a.out_vals[base + a.heads[u] - 1] = __longlong_as_double((long long)Op::finalize(last_of[u], L));
+    if (bad) atomicOr(a.inexact, 1u);
   }
 }
 
@@ -672,101 +698,94 @@ __global__ void sum_u32_kernel(const uint32_t* v, uint64_t n, uint32_t* out) {
 }
 
 // ------------------------------------------------------------------ host side
+// Elements per unit: one unit per resident warp of the main pass where that gives full units
+// (32 warps on each of 148 SMs), fewer elements for short inputs.
+uint32_t f64_unit_items(uint64_t n) {
+  const uint64_t per = (n + 32 * 148 - 1) / (32 * 148);
+  const uint64_t steps = (per + kF64Step - 1) / kF64Step;
+  return (uint32_t)(steps * kF64Step < kF64UnitMost ? steps * kF64Step : kF64UnitMost);
+}
+
+// done, the exponent maximum and the two passes' flags (cleared), then the counts and first run
+// indices, which every pass shares, then the partials of the pass that runs.
 struct F64Layout {
-  size_t total = 0;
-  uint64_t* status = nullptr;
-  uint32_t* counter = nullptr;
-  uint32_t* tile_heads = nullptr;
-  uint32_t* tile_base = nullptr;
-  void* tile_first = nullptr;
-  void* tile_last = nullptr;
-  void* exc = nullptr;
-  void* chunk_agg = nullptr;
-  int* emax = nullptr;
-  uint32_t* inexact = nullptr;
-  size_t clear = 0;  // bytes from the start to zero before a launch
+  uint32_t* done;
+  int* emax;
+  uint32_t* inexact_pair;
+  uint32_t* inexact_narrow;
+  size_t clear;
+  uint32_t* heads;
+  uint32_t* base;
+  uint8_t* first;
+  uint8_t* last;
+  size_t total;
 };
 
-template <class Op>
-F64Layout f64_layout(void* ws, uint64_t n, uint64_t tile_items) {
-  using P = typename Op::P;
-  const uint64_t tiles = (n + tile_items - 1) / tile_items;
-  const uint64_t chunks = (tiles + kFixThreads - 1) / kFixThreads;
+F64Layout f64_layout(void* ws, uint64_t n) {
+  const uint64_t unit = f64_unit_items(n), units = unit ? (n + unit - 1) / unit : 0;
+  constexpr size_t partial = sizeof(SumOp<kWideLimbs>::P);   // the largest
+  static_assert(partial % 16 == 0 || partial % 8 == 0, "aligned partials");
   F64Layout l;
   Carver c(ws);
-  l.status = c.take<uint64_t>(tiles + 1);
-  l.counter = c.take<uint32_t>(4);
-  l.emax = c.take<int>(4);
-  l.inexact = c.take<uint32_t>(4);
-  l.clear = c.used;
-  l.tile_heads = c.take<uint32_t>(tiles + 1);
-  l.tile_base = c.take<uint32_t>(tiles + 1);
-  l.tile_first = c.take<P>(tiles + 1);
-  l.tile_last = c.take<P>(tiles + 1);
-  l.exc = c.take<Seg<P>>(tiles + 1);
-  l.chunk_agg = c.take<Seg<P>>(chunks + 1);
-  l.total = c.used + 256;
+  uint32_t* words = c.take<uint32_t>(4);
+  l.done = words;
+  l.emax = reinterpret_cast<int*>(words) + 1;
+  l.inexact_pair = words + 2;
+  l.inexact_narrow = words + 3;
+  l.clear = 4 * sizeof(uint32_t);
+  l.heads = c.take<uint32_t>(units + 1);
+  l.base = c.take<uint32_t>(units + 1);
+  l.first = c.take<uint8_t>((units + 1) * partial);
+  l.last = c.take<uint8_t>((units + 1) * partial);
+  l.total = align_up(c.used + 256, 256);
   return l;
 }
 
-size_t f64_core(uint64_t n) {
-  const size_t a = f64_layout<SumOp<kNarrowLimbs>>(nullptr, n, kF64UnitItems).total;
-  const size_t b = f64_layout<SumOp<kWideLimbs>>(nullptr, n, kF64UnitItems).total;
-  const size_t c = f64_layout<MinOp>(nullptr, n, kF64UnitItems).total;
-  return align_up(a > b ? (a > c ? a : c) : (b > c ? b : c), 256);
-}
+size_t f64_workspace(uint64_t n) { return f64_layout(nullptr, n).total; }
 
-// The layouts, then one word past them: the narrow pass's inexact flag, which gates the
-// full-range pass.
-size_t f64_workspace(uint64_t n) { return f64_core(n) + 256; }
-
-// The unit path: count + scan, one warp per unit, then the tile fix-up over units.
+// One pass over the units and its fix-up.
 template <int KB, class Op>
-rfx_status f64_run_units(F64Args a, void* ws, bool narrow_sum, int fixed_L, cudaStream_t s) {
-  const F64Layout l = f64_layout<Op>(ws, a.n, kF64UnitItems);
-  RFX_CUDA_TRY(cudaMemsetAsync(ws, 0, l.clear, s));
-  a.status = l.status;
-  a.counter = l.counter;
-  a.tile_heads = l.tile_heads;
-  a.tile_base = l.tile_base;
-  a.tile_first = l.tile_first;
-  a.tile_last = l.tile_last;
-  a.exc = l.exc;
-  a.chunk_agg = l.chunk_agg;
-  a.inexact = l.inexact;
-  a.d_emax = narrow_sum ? l.emax : nullptr;
-  a.fixed_L = fixed_L;
-  const uint64_t units = (a.n + kF64UnitItems - 1) / kF64UnitItems;
-  const uint64_t chunks = (units + kFixThreads - 1) / kFixThreads;
+rfx_status f64_run_units(const F64Args& a, uint64_t units, cudaStream_t s) {
   const uint64_t want = (units + 7) / 8;
-  const int gc = persistent_grid((const void*)f64_unit_count<KB>, 256, 0, want);
-  f64_unit_count<KB><<<gc, 256, 0, s>>>(a, units, narrow_sum ? l.emax : nullptr);
-  RFX_CUDA_TRY(cudaGetLastError());
-  f64_unit_scan<<<1, 1024, 0, s>>>(a, units);
-  RFX_CUDA_TRY(cudaGetLastError());
   const int gm = persistent_grid((const void*)f64_unit_kernel<KB, Op>, 256, 0, want);
   f64_unit_kernel<KB, Op><<<gm, 256, 0, s>>>(a, units);
   RFX_CUDA_TRY(cudaGetLastError());
-  f64_fix_scan<Op><<<(int)chunks, kFixThreads, 0, s>>>(a, units);
-  RFX_CUDA_TRY(cudaGetLastError());
-  f64_fix_chunks<Op><<<1, kFixThreads, 0, s>>>(a, chunks);
-  RFX_CUDA_TRY(cudaGetLastError());
-  f64_fix_apply<Op><<<(int)chunks, kFixThreads, 0, s>>>(a, units);
+  f64_fix<Op><<<(int)want, 256, 0, s>>>(a, units);
   RFX_CUDA_TRY(cudaGetLastError());
   return RFX_OK;
 }
 
 template <int KB>
 rfx_status f64_dispatch_op(F64Args a, uint32_t op, void* ws, cudaStream_t s) {
-  if (op == RFX_F64_MIN) return f64_run_units<KB, MinOp>(a, ws, false, 0, s);
-  rfx_status st = f64_run_units<KB, SumOp<kNarrowLimbs>>(a, ws, true, 0, s);
+  const F64Layout l = f64_layout(ws, a.n);
+  a.unit = f64_unit_items(a.n);
+  const uint64_t units = (a.n + a.unit - 1) / a.unit;
+  a.done = l.done;
+  a.heads = l.heads;
+  a.base = l.base;
+  a.first = l.first;
+  a.last = l.last;
+  a.inexact = l.inexact_pair;
+  RFX_CUDA_TRY(cudaMemsetAsync(ws, 0, l.clear, s));
+  const int gc = persistent_grid((const void*)f64_unit_count<KB>, 256, 0, (units + 7) / 8);
+  f64_unit_count<KB><<<gc, 256, 0, s>>>(a, units);
+  RFX_CUDA_TRY(cudaGetLastError());
+  if (op == RFX_F64_MIN) return f64_run_units<KB, MinOp>(a, units, s);
+  rfx_status st = f64_run_units<KB, PairOp>(a, units, s);
   if (st != RFX_OK) return st;
-  // the full-range pass runs on the device only if the narrow window lost bits
-  const F64Layout l = f64_layout<SumOp<kNarrowLimbs>>(ws, a.n, kF64UnitItems);
-  uint32_t* gate = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(ws) + f64_core(a.n));
-  RFX_CUDA_TRY(cudaMemcpyAsync(gate, l.inexact, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-  a.gate = gate;
-  return f64_run_units<KB, SumOp<kWideLimbs>>(a, ws, false, kWideL, s);
+  // each further pass runs on the device only if the one before lost bits
+  a.gate = l.inexact_pair;
+  a.inexact = l.inexact_narrow;
+  a.emax = l.emax;
+  const int ge = persistent_grid((const void*)f64_emax, 256, 0, (a.n + 2047) / 2048);
+  f64_emax<<<ge, 256, 0, s>>>(a);
+  RFX_CUDA_TRY(cudaGetLastError());
+  st = f64_run_units<KB, SumOp<kNarrowLimbs>>(a, units, s);
+  if (st != RFX_OK) return st;
+  a.gate = l.inexact_narrow;
+  a.emax = nullptr;
+  a.fixed_L = kWideL;
+  return f64_run_units<KB, SumOp<kWideLimbs>>(a, units, s);
 }
 
 rfx_status f64_dispatch(F64Args a, uint32_t key_bytes, uint32_t op, void* ws, cudaStream_t s) {

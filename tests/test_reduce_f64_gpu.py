@@ -221,3 +221,29 @@ def test_total_string_double(cuda):
     assert g == es.shape[0] and int(vs.item()) // 8 == g
     assert np.array_equal((to_np(ok[:g]) - dpool.data_ptr()).astype(np.uint64), eo)
     assert _same_bits(to_np(ov[:g]), es)
+
+
+@pytest.mark.parametrize("n,groups", [(255, 1), (255, 1 << 30), (256, 40), (257, 1), (257, 1 << 30), (1025, 40),
+                                      (4737 * 256 + 5, 1000)])
+def test_sum_unit_edges_and_passes(cuda, n, groups):
+    """Units of one and two 256-element steps and their edges, one run over all, runs of a few
+    elements and of one; amounts (the pair of doubles stays exact), a span that needs the
+    integer pass, and unaligned columns."""
+    keys = gen_keys(4, n, min(groups, 2 * n), n)
+    for kind in ("prices", "mixed"):
+        vals = gen_values(kind, n, n + 1)
+        _check_sum(cuda, keys, vals)
+        if n > 300:
+            dk, dv = _dev(keys, cuda)[1:], _dev(vals, cuda)[1:]
+            ok, ov, g = R.reduce_f64(dk, dv, R.F64_SUM)
+            ek, es = O.reduce_f64_exact(keys[1:], vals[1:])
+            assert g == es.shape[0] and np.array_equal(to_np(ok), ek) and _same_bits(to_np(ov), es)
+
+
+def test_sum_pair_signs_and_cancellation(cuda):
+    """Zeros keep IEEE's sign (-0 only when every term is), sums that cancel are +0, a sum of
+    2^53 and odd terms rounds once."""
+    vals = np.array([-0.0, -0.0, -0.0, 0.0, 5.0, -5.0, -0.0, 2.0**53, 1.0, 1.0, 2.0**53, 1.0, -2.0**53, 2.0**-40],
+                    np.float64)
+    keys = np.array([0, 0, 1, 1, 2, 2, 2, 3, 3, 3, 4, 4, 5, 5], np.uint32)
+    _check_sum(cuda, keys, vals)
