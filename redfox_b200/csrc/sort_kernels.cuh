@@ -21,16 +21,16 @@ constexpr int kSortLookWindow = 8;  // predecessors examined per look-back round
 // The tile of a digit pass by the bytes of a key and its value.  Two blocks per SM: as large
 // a tile as their shared memory allows (the per-tile costs -- barriers, the look-back -- and
 // the number of digit runs a tile is written in fall with its size), over as many threads as
-// that leaves registers for.  60M keys, us per pass, of the shapes tried:
-//   4 B   512 x 20 and 384 x 24: 212; 512 x 16, 384 x 16 with 3 blocks: 218; 512 x 12: 241
-//   8 B   384 x 16: 274; 512 x 12: 277; 512 x 8: 335
-//   16 B  512 x 8: 407; 384 x 10: 422; 1024 x 8, one block: 436
-//   4 B keys with 8 B values (4M): 384 x 12: 31.5; 512 x 8: 35.1; 512 x 12, one block: 37.6
+// that leaves registers for.  Whole sorts of four passes, us, at 1M / 4M / 60M elements:
+//   4 B   512 x 20: 63 / 117 / 942; 512 x 22: 68 / 122 / 930; 384 x 28: 74 / 133 / 1060
+//   8 B   512 x 14: 62 / 120 / 1170; 512 x 12: 62 / 125 / 1211; 384 x 16: 62 / 138 / 1281
+//   4 B keys with 8 B values   512 x 10: 65 / 141 / 1447; 384 x 12: 63 / 148 / 1510; 384 x 16: 71 / 153 / 1389
+//   16 B  512 x 9: 67 / 162 / 1688; 512 x 8: 65 / 166 / 1746; 384 x 12: 71 / 167 / 1710
 template <int K, int V>
 struct SortTuning {
   static constexpr int B = K + V;
-  static constexpr int THREADS = B <= 4 ? 512 : B <= 12 ? 384 : B <= 16 ? 512 : B <= 48 ? 384 : 256;
-  static constexpr int IPT = B <= 4 ? 20 : B <= 8 ? 16 : B <= 12 ? 12 : B <= 16 ? 8 : B <= 32 ? 6 : 4;
+  static constexpr int THREADS = B <= 16 ? 512 : B <= 48 ? 384 : 256;
+  static constexpr int IPT = B <= 4 ? 20 : B <= 8 ? 14 : B <= 12 ? 10 : B <= 16 ? 9 : B <= 32 ? 6 : 4;
   static constexpr int WARPS = THREADS / 32;
   static constexpr int TILE = THREADS * IPT;
   // dynamic shared memory: the tile's keys and values as they lie in global memory, every
@@ -184,9 +184,10 @@ __device__ __forceinline__ void st_relaxed_u32(uint32_t* p, uint32_t v) {
 //
 // Every lane counts in bins of its own (bin d of lane l at word d * 32 + l, so that the 32
 // lanes always hit 32 banks): a digit is two or three instructions and one wavefront,
-// whatever its distribution.  Bins shared by the block, with a warp vote that took digits
-// equal in all lanes together, were bound by instruction issue and bank conflicts: 60M
-// 4-byte keys with four digits 337 us, 60M 16-byte rows 483 us.  16 bytes per load and
+// whatever its distribution; one funnel shift brings a group's digits into one word.  Bins
+// shared by the block, with a warp vote that took digits equal in all lanes together, were
+// bound by instruction issue and bank conflicts: 60M 4-byte keys with four digits 337 us (now
+// 60), 60M 16-byte rows 483 us (178).  16 bytes per load and
 // thread, kHistLoads loads in flight.
 constexpr int kHistThreads = 1024;
 constexpr int kHistPlaces = 4;
@@ -198,28 +199,43 @@ __device__ __forceinline__ void hist_count(uint32_t at) {
   asm volatile("red.shared.add.u32 [%0 + %1], 1;" ::"r"(at), "n"(PLACE * kHistPlaceBytes) : "memory");
 }
 
+// The 32 bits of an element from bit `begin` on hold every digit of a group of up to four
+// places; digit p is bits [8 p, 8 p + 8) of them.
 template <int K, int P>
 struct HistDigits {
-  uint32_t shift[P];   // first bit of each place's digit (single words: the rotation that brings it to bit 7)
-  uint32_t mask[P];    // the digit's mask, at bit 7
+  uint32_t q, sh;      // the word and the bit in it where the group's digits begin
+  uint32_t mask[P];    // each place's digit mask, at bit 7
   uint32_t at;         // this lane's bin 0 of place 0
   __device__ __forceinline__ HistDigits(uint32_t bins, uint32_t begin, uint32_t end) : at(bins + (threadIdx.x & 31) * 4) {
+    q = begin >> 5;
+    sh = begin & 31;
 #pragma unroll
     for (int p = 0; p < P; ++p) {
       const uint32_t s = begin + 8 * p;
       const uint32_t w = s >= end ? 0u : end - s < 8 ? end - s : 8u;   // places past the last pass: digit 0
-      shift[p] = Elem<K>::NW == 1 ? (s - 7) & 31 : min(s, 8u * K - 1);
       mask[p] = ((1u << w) - 1) << 7;
     }
   }
   template <int PLACE = 0>
-  __device__ __forceinline__ void count(const Elem<K>& e) const {
+  __device__ __forceinline__ void count_places(uint32_t w) const {
     if constexpr (PLACE < P) {
-      uint32_t x;
-      if constexpr (Elem<K>::NW == 1) x = __funnelshift_r(e.w[0], e.w[0], shift[PLACE]);
-      else x = elem_bits<K>(e, shift[PLACE]) << 7;
-      hist_count<PLACE>(at + (x & mask[PLACE]));
-      count<PLACE + 1>(e);
+      hist_count<PLACE>(at + (__funnelshift_r(w, w, (8 * PLACE - 7) & 31) & mask[PLACE]));
+      count_places<PLACE + 1>(w);
+    }
+  }
+  __device__ __forceinline__ void count(const Elem<K>& e) const {
+    if constexpr (Elem<K>::NW == 1) {
+      count_places(e.w[0] >> sh);
+    } else {
+      uint32_t lo = e.w[0], hi = e.w[1];
+#pragma unroll
+      for (int k = 1; k < Elem<K>::NW; ++k) {
+        if ((int)q == k) {
+          lo = e.w[k];
+          hi = k + 1 < Elem<K>::NW ? e.w[k + 1] : 0u;
+        }
+      }
+      count_places(__funnelshift_r(lo, hi, sh));
     }
   }
 };
@@ -348,7 +364,7 @@ sort_histogram_kernel(const uint8_t* __restrict__ keys, uint64_t n, uint32_t beg
 // for its block's current one, and every later tile's look-back waits for it, so all
 // blocks ran at the pace of the slowest.  A tile is now claimed while the one before it is
 // written out, and what a block will claim about a round later is brought into L2 by a
-// prefetch.  60M keys, us per pass, before -> now: 4 B 325 -> 212, 8 B 430 -> 274, 16 B 605 -> 407.
+// prefetch.  60M keys, us per pass, before -> now: 4 B 325 -> 220, 8 B 430 -> 270, 16 B 605 -> 385.
 //
 // Stability.  The order in which one atomic instruction serves the lanes that share a digit
 // is not specified, so the keys of one warp step may come out exchanged.  Entries must
@@ -388,6 +404,15 @@ __device__ __forceinline__ uint32_t sort_lookback(const uint32_t* status, uint32
     } else {
 #pragma unroll
       for (int r = 0; r < kSortLookWindow; ++r) w[r] = r <= base ? ld_relaxed_u32(p - r * kRadix) : kSFlagInc;
+    }
+    // the whole window ready and none inclusive, as in most rounds but a tile's last: the
+    // flags of eight words (2^30 each) add up to a multiple of 2^32
+    static_assert(kSortLookWindow == 8, "see above");
+    const uint32_t all = w[0] & w[1] & w[2] & w[3] & w[4] & w[5] & w[6] & w[7];
+    if (all & kSFlagAgg) {
+      prefix += ((w[0] + w[1]) + (w[2] + w[3])) + ((w[4] + w[5]) + (w[6] + w[7]));
+      base -= kSortLookWindow;
+      continue;
     }
     bool open = true, done = false;
     uint32_t used = 0;
@@ -580,15 +605,8 @@ sort_pass_kernel(const __grid_constant__ SortPassArgs a) {
     for (int j = 0; j < IPT; ++j)
       if (full || (uint32_t)j < nv)
         entries[wcount[key[j] >> 16] + (key[j] & 0xffffu)] = (key[j] & 0xffff0000u) | (first + j * 32);
-    if (t < kRadix) {
-      uint32_t prefix = gexcl;
-      if (tile > 0) {
-        prefix = sort_lookback(a.status, tile, a.err);
-        st_relaxed_u32(status, kSFlagInc | ((prefix + count) & kSValMask));
-      }
-      s_base[t] = prefix - start;
-    }
     __syncthreads();
+    // the look-back comes last before the write-out, which gives the predecessors that long
     for (uint32_t k = t; k < T::COUNTERS / 16; k += THREADS)
       reinterpret_cast<uint4*>(counters)[k] = make_uint4(0, 0, 0, 0);
     uint32_t entry[IPT];
@@ -598,6 +616,14 @@ sort_pass_kernel(const __grid_constant__ SortPassArgs a) {
       const uint32_t i = j * THREADS + t;
       entry[j] = entries[i];
       disorder = disorder || (i > 0 && i < tcount && entries[i - 1] > entry[j]);
+    }
+    if (t < kRadix) {
+      uint32_t prefix = gexcl;
+      if (tile > 0) {
+        prefix = sort_lookback(a.status, tile, a.err);
+        st_relaxed_u32(status, kSFlagInc | ((prefix + count) & kSValMask));
+      }
+      s_base[t] = prefix - start;
     }
     if (__syncthreads_or(disorder)) {
       order_entries(entries, tcount, THREADS);

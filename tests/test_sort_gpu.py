@@ -216,17 +216,19 @@ def test_sort_from_all_trivial_and_overlap(cuda):
 
 
 # Keys per tile of the digit pass, by key and value bytes (SortTuning): 4 B 10240, up to 8 B
-# 6144, up to 12 B 4608, up to 16 B 4096, up to 32 B 2304, up to 48 B 1536, above 1024.
-TILE_KEYS = {(1, 0): 10240, (4, 0): 10240, (8, 0): 6144, (4, 4): 6144, (4, 8): 4608, (16, 0): 4096, (8, 8): 4096,
+# 7168, up to 12 B 5120, up to 16 B 4608, up to 32 B 2304, up to 48 B 1536, above 1024.
+TILE_KEYS = {(1, 0): 10240, (4, 0): 10240, (8, 0): 7168, (4, 4): 7168, (4, 8): 5120, (16, 0): 4608, (8, 8): 4608,
              (16, 16): 2304, (32, 0): 2304, (32, 16): 1536, (64, 16): 1024}
+ABOVE_CLUSTER = 70_000   # rows the one-launch sort does not take
 
 
 @pytest.mark.parametrize("kb,vb", sorted(TILE_KEYS))
 @pytest.mark.parametrize("extra", [-1, 0, 1, 2 * 10240 + 17])
 def test_sort_tile_edges_with_many_equal_digits(cuda, kb, vb, extra):
-    """One tile less a key, a whole tile, a key more, a few tiles; digits that straddle a
+    """Whole tiles less a key, whole tiles, a key more, some tiles more; digits that straddle a
     32-bit word and digits that most of a warp's keys share, whose order must stay."""
-    n = TILE_KEYS[kb, vb] + extra
+    tile = TILE_KEYS[kb, vb]
+    n = (ABOVE_CLUSTER // tile + 1) * tile + extra
     keys = _keys(n, kb, seed=n + kb)
     keys[:, (kb * 8 - 5) // 8] &= np.uint8(0x13)
     vals = np.random.default_rng(n).integers(0, 256, (n, vb), dtype=np.uint8) if vb else None
