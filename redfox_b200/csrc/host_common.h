@@ -46,6 +46,24 @@ inline cudaStream_t as_stream(void* s) { return static_cast<cudaStream_t>(s); }
 int persistent_grid(const void* kernel, int threads, size_t dyn_smem, uint64_t work_blocks);
 // Raise a kernel's dynamic shared memory limit once.
 cudaError_t allow_smem(const void* kernel, size_t bytes);
+// Launches a kernel that calls grid_wait() before it touches memory: its launch and its
+// blocks' start overlap the end of the kernel before it in the stream.
+template <typename... Params, typename... Args>
+cudaError_t launch_chained(void (*kernel)(Params...), int grid, int threads, size_t dyn_smem, cudaStream_t stream,
+                           Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = dyn_smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // Whether a cluster of `blocks` blocks of the kernel can be resident on the current device
 // (looked up once per device, kernel, cluster size and shared memory); raises the kernel's
 // limits on shared memory and cluster size.

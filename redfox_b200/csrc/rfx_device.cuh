@@ -52,6 +52,13 @@ __device__ __forceinline__ void block_prefetch16(uint8_t* dst, const uint8_t* sr
   }
 }
 
+// Programmatic dependent launch: a kernel launched with launch_chained (host_common.h) may
+// start while the kernel before it in the stream still runs; grid_wait() holds it until that
+// one has completed and its writes are visible.  grid_release() lets the next kernel's blocks
+// take the resources that become free.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ------------------------------------------------------------------ memory order
 __device__ __forceinline__ uint64_t ld_relaxed_u64(const uint64_t* p) {
   uint64_t v;

@@ -26,11 +26,22 @@ constexpr int kSortLookWindow = 8;  // predecessors examined per look-back round
 //   8 B   512 x 14: 62 / 120 / 1170; 512 x 12: 62 / 125 / 1211; 384 x 16: 62 / 138 / 1281
 //   4 B keys with 8 B values   512 x 10: 65 / 141 / 1447; 384 x 12: 63 / 148 / 1510; 384 x 16: 71 / 153 / 1389
 //   16 B  512 x 9: 67 / 162 / 1688; 512 x 8: 65 / 166 / 1746; 384 x 12: 71 / 167 / 1710
+// Inputs of fewer large tiles than SMs take small tiles instead (elements of 4 to 16 bytes):
+// a tile's chain is shorter and more SMs work.  Large -> small, us:
+//   4 B   100K 51 -> 38, 1M (98 large tiles) 61 -> 52, 2M (196) 70 -> 75
+//   8 B   300K 48 -> 42, 1M (140) 59 -> 58, 2M (280) 67 -> 84
+//   16 B  100K 42 -> 36, 300K (66) 46 -> 44, 1M (218) 62 -> 71
+constexpr uint64_t kSortSmallBelow = 148;   // large tiles
+
 template <int K, int V>
+constexpr bool kSortHasSmall = (K == 4 || K == 8 || K == 16) && K + V <= 16;
+
+template <int K, int V, bool SMALL = false>
 struct SortTuning {
   static constexpr int B = K + V;
   static constexpr int THREADS = B <= 16 ? 512 : B <= 48 ? 384 : 256;
-  static constexpr int IPT = B <= 4 ? 20 : B <= 8 ? 14 : B <= 12 ? 10 : B <= 16 ? 9 : B <= 32 ? 6 : 4;
+  static constexpr int LARGE = B <= 4 ? 20 : B <= 8 ? 14 : B <= 12 ? 10 : B <= 16 ? 9 : B <= 32 ? 6 : 4;
+  static constexpr int IPT = !SMALL ? LARGE : B <= 4 ? 8 : B <= 8 ? 6 : B <= 12 ? 5 : 4;
   static constexpr int WARPS = THREADS / 32;
   static constexpr int TILE = THREADS * IPT;
   // dynamic shared memory: the tile's keys and values as they lie in global memory, every
@@ -277,6 +288,7 @@ sort_histogram_kernel(const uint8_t* __restrict__ keys, uint64_t n, uint32_t beg
   __shared__ uint32_t s_moving;   // bit p: pass p has more than one digit
   const uint32_t t = threadIdx.x, lane = t & 31;
   const uint64_t tid = (uint64_t)blockIdx.x * kHistThreads + t, stride = (uint64_t)gridDim.x * kHistThreads;
+  grid_release();
   for (uint64_t k = tid; k < status_chunks; k += stride) status[k] = make_uint4(0, 0, 0, 0);
   // whole 16-byte chunks where the elements tile them; the rest element by element
   const bool vec = K <= 16 && (reinterpret_cast<uintptr_t>(keys) & 15u) == 0;
@@ -473,10 +485,10 @@ __device__ void grid_copy(uint8_t* dst, const uint8_t* src, uint64_t n) {
   for (uint64_t i = chunks * 16 / B + tid; i < n; i += stride) store_elem<B>(dst, i, load_elem<B>(src, i));
 }
 
-template <int K, int V>
-__global__ void __launch_bounds__((SortTuning<K, V>::THREADS), 2)
+template <int K, int V, bool SMALL>
+__global__ void __launch_bounds__((SortTuning<K, V, SMALL>::THREADS), 2)
 sort_pass_kernel(const __grid_constant__ SortPassArgs a) {
-  using T = SortTuning<K, V>;
+  using T = SortTuning<K, V, SMALL>;
   constexpr int IPT = T::IPT, WARPS = T::WARPS;
   constexpr uint32_t TILE = T::TILE, THREADS = T::THREADS;
   extern __shared__ __align__(16) uint8_t sbuf[];
@@ -489,6 +501,14 @@ sort_pass_kernel(const __grid_constant__ SortPassArgs a) {
   __shared__ uint32_t s_tile;
   __shared__ __align__(8) uint64_t s_bar;
   const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  // chained launch: what needs no other kernel's results comes before the wait
+  if (t == 0) {
+    mbar_init(&s_bar, 1);
+    mbar_fence_init();
+  }
+  for (uint32_t k = t; k < T::COUNTERS / 16; k += THREADS) reinterpret_cast<uint4*>(counters)[k] = make_uint4(0, 0, 0, 0);
+  grid_wait();
+  grid_release();
   const uint32_t route = *a.route;
   const uint32_t n = (uint32_t)a.n;   // below 2^30
   const uint32_t num_tiles = (n + TILE - 1) / TILE;
@@ -496,14 +516,9 @@ sort_pass_kernel(const __grid_constant__ SortPassArgs a) {
   const bool straddle = sh + (32 - __clz(mask)) > 32;
   uint32_t* const wcount = counters + warp * kRadix;
   const uint32_t gexcl = t < kRadix ? a.gexcl[t] : 0u;
-  // a tile is claimed (and the counters cleared) while the route is on its way; a pass that
-  // turns out not to sort has no use for its tile numbers
-  if (t == 0) {
-    mbar_init(&s_bar, 1);
-    mbar_fence_init();
-    s_tile = atomicAdd(a.tile_counter, 1u);
-  }
-  for (uint32_t k = t; k < T::COUNTERS / 16; k += THREADS) reinterpret_cast<uint4*>(counters)[k] = make_uint4(0, 0, 0, 0);
+  // a tile is claimed while the route is on its way; a pass that turns out not to sort has no
+  // use for its tile numbers
+  if (t == 0) s_tile = atomicAdd(a.tile_counter, 1u);
   __syncthreads();
   // the buffers are looked up in the parameters where they are used, which leaves no register
   // to their addresses

@@ -41,9 +41,16 @@ struct ClusterSort {
   cudaStream_t stream;
 };
 
+// Whether n elements take the pass's small tiles, and how many tiles they make.
+template <int K, int V>
+bool sort_small(uint64_t n) {
+  return kSortHasSmall<K, V> && n <= kSortSmallBelow * SortTuning<K, V>::TILE;
+}
+
 template <int K, int V>
 uint64_t sort_tiles(uint64_t n) {
-  return (n + SortTuning<K, V>::TILE - 1) / SortTuning<K, V>::TILE;
+  const uint64_t tile = sort_small<K, V>(n) ? SortTuning<K, V, kSortHasSmall<K, V>>::TILE : SortTuning<K, V>::TILE;
+  return (n + tile - 1) / tile;
 }
 
 // Histogram of every digit; clears the look-back words.
@@ -61,17 +68,13 @@ rfx_status launch_histogram(SortPlan& s) {
   return RFX_OK;
 }
 
-template <int K, int V>
-rfx_status run_sort_kv(SortPlan& s) {
-  rfx_status hst = s.passes == 1   ? launch_histogram<K, 1>(s)
-                   : s.passes == 2 ? launch_histogram<K, 2>(s)
-                   : s.passes == 3 ? launch_histogram<K, 3>(s)
-                                   : launch_histogram<K, kHistPlaces>(s);
-  if (hst != RFX_OK) return hst;
-  auto pass = sort_pass_kernel<K, V>;
-  constexpr size_t smem = SortTuning<K, V>::SMEM;
+template <int K, int V, bool SMALL>
+rfx_status run_passes(SortPlan& s) {
+  using T = SortTuning<K, V, SMALL>;
+  auto pass = sort_pass_kernel<K, V, SMALL>;
+  constexpr size_t smem = T::SMEM;
   RFX_CUDA_TRY(allow_smem((const void*)pass, smem));
-  const int grid = persistent_grid((const void*)pass, SortTuning<K, V>::THREADS, smem, s.tiles);
+  const int grid = persistent_grid((const void*)pass, T::THREADS, smem, s.tiles);
   for (uint32_t p = 0; p < s.passes; ++p) {
     SortPassArgs a;
     a.keys[0] = s.src_keys ? const_cast<uint8_t*>(s.src_keys) : s.keys;   // out of place: never written
@@ -91,10 +94,22 @@ rfx_status run_sort_kv(SortPlan& s) {
     a.status = s.status + (uint64_t)p * s.tiles * kRadix;
     a.tile_counter = s.counters + p;
     a.err = s.err;
-    pass<<<grid, SortTuning<K, V>::THREADS, smem, s.stream>>>(a);
-    RFX_CUDA_TRY(cudaGetLastError());
+    RFX_CUDA_TRY(launch_chained(pass, grid, T::THREADS, smem, s.stream, a));
   }
   return RFX_OK;
+}
+
+template <int K, int V>
+rfx_status run_sort_kv(SortPlan& s) {
+  rfx_status hst = s.passes == 1   ? launch_histogram<K, 1>(s)
+                   : s.passes == 2 ? launch_histogram<K, 2>(s)
+                   : s.passes == 3 ? launch_histogram<K, 3>(s)
+                                   : launch_histogram<K, kHistPlaces>(s);
+  if (hst != RFX_OK) return hst;
+  if constexpr (kSortHasSmall<K, V>) {
+    if (sort_small<K, V>(s.n)) return run_passes<K, V, true>(s);
+  }
+  return run_passes<K, V, false>(s);
 }
 
 // The one-launch sort of small inputs; RFX_ERR_UNSUPPORTED when it does not take this one

@@ -291,3 +291,23 @@ def test_sort_small_inputs_in_one_cluster(cuda, kb, vb, most, n):
             if vb:
                 assert np.array_equal(to_np(v), exp[1]), (begin, end)
     assert R.device_status() == R.OK
+
+
+@pytest.mark.parametrize("kb,vb", [(4, 0), (8, 0), (4, 4), (4, 8), (8, 4), (16, 0), (8, 8)])
+@pytest.mark.parametrize("where", ["small tile", "last small", "first large"])
+def test_sort_small_and_large_tiles(cuda, kb, vb, where):
+    """The pass's small tiles (512 threads x 8, 6, 5 or 4 elements) at a tile's edge, the most
+    elements that take them (148 large tiles) and one more."""
+    small = 512 * {4: 8, 8: 6, 12: 5, 16: 4}[kb + vb]
+    n = {"small tile": (ABOVE_CLUSTER // small + 1) * small + 1, "last small": 148 * TILE_KEYS.get((kb, vb), 5120),
+         "first large": 148 * TILE_KEYS.get((kb, vb), 5120) + 1}[where]
+    keys = _keys(n, kb, seed=n + kb)
+    vals = np.random.default_rng(n).integers(0, 256, (n, vb), dtype=np.uint8) if vb else None
+    begin, end = kb * 8 - 19, kb * 8
+    dk, dv = R.sorted_copy(_dev(keys, cuda), _dev(vals, cuda) if vb else None, begin_bit=begin, end_bit=end)
+    exp = (O.sort_pairs(keys, vals, begin_bit=begin, end_bit=end, threads=8) if vb
+           else (O.sort_pairs(keys, begin_bit=begin, end_bit=end, threads=8), None))
+    assert np.array_equal(to_np(dk), exp[0])
+    if vb:
+        assert np.array_equal(to_np(dv), exp[1])
+    assert R.device_status() == R.OK
