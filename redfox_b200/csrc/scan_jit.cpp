@@ -358,8 +358,8 @@ std::string gen_compact(const ScanProgram& p, int mode, uint32_t wout, int rows_
   const int no = limbs(wout);
   std::ostringstream s;
   s << kPreamble;
-  s << "#define NT " << kJitThreads << "\n#define NL " << nl << "\n#define NO " << no << "\n#define IPT "
-    << rows_per_thread << "\n#define TILE (NT * IPT)\n";
+  s << "#define NT " << kJitThreads << "\n#define NL " << nl << "\n#define NO " << no << "\n#define ROWB "
+    << p.in_bytes << "\n#define EARLY " << (mode == 1) << "\n#define IPT " << rows_per_thread << "\n#define TILE (NT * IPT)\n";
   s << "static __device__ __forceinline__ bool process(const u64 (&L)[NL], u64 (&O)[NO], const RfxConsts& K) {\n";
   s << row_body(p, "L");
   if (mode == 0) {
@@ -409,7 +409,11 @@ extern "C" __global__ void __launch_bounds__(NT) rfx_plan_compact(
   // look-back; then all warps write tile k's staged rows out as one contiguous run.  No
   // look-back stands between a claim and that tile's count, a tile is resolved a whole
   // step after its count was published, and the look-back's L2 round trips overlap the
-  // next tile's loads.
+  // next tile's loads.  The rows that some block claims about a round later are prefetched
+  // into L2.  EARLY (projections): the next tile is claimed during the write-out.  20M rows of
+  // 64 bytes, us a call at 8 / 48 / 98 % kept: select 408 / 512 / 643 -> 383 / 485 / 623 (with
+  // EARLY 436 / 518 / 634); select + project to 32 bytes 384 / 423 / 451 -> 340 / 365 / 405
+  // (without EARLY 351 / 377 / 421).
   s << R"RFX(
 #define NTB (NT + 32)
 extern "C" __global__ void __launch_bounds__(NTB) rfx_plan_compact(
@@ -420,15 +424,22 @@ extern "C" __global__ void __launch_bounds__(NTB) rfx_plan_compact(
   __shared__ u32 s_total[2];
   __shared__ u32 s_tile[2];
   __shared__ u64 s_prefix;
+  __shared__ u32 s_next;   // the claimed tile that fill() takes next
   const u32 t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const u64 num_tiles = (n + TILE - 1) / TILE;
+  if (EARLY && t == 0) s_next = atomicAdd(tile_counter, 1u);
+  __syncthreads();
   // compute warps only (barrier 1 over NT threads): claim, load, evaluate, rank and
   // stage one tile into buffer b; publish its count
   auto fill = [&](int b) {
-    if (t == 0) s_tile[b] = atomicAdd(tile_counter, 1u);
+    if (t == 0) s_tile[b] = EARLY ? s_next : atomicAdd(tile_counter, 1u);
     asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
     const u64 tile = s_tile[b];
     if (tile >= num_tiles) return;
+    // what some block claims about a round from now, into L2
+    const u64 ahead = (tile + gridDim.x) * TILE;
+    if (t == 0 && ahead + TILE <= n && ((unsigned long long)in & 15u) == 0)
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(in + ahead * ROWB), "r"((u32)(TILE * ROWB)) : "memory");
     u64 L[IPT][NL];
 #pragma unroll
     for (int j = 0; j < IPT; ++j) {
@@ -481,6 +492,8 @@ extern "C" __global__ void __launch_bounds__(NTB) rfx_plan_compact(
   if (t < NT) fill(0);
   __syncthreads();
   u64 tc = s_tile[0];
+  if (EARLY && t == 0) s_next = atomicAdd(tile_counter, 1u);
+  __syncthreads();
   for (int b = 0; tc < num_tiles; b ^= 1) {
     if (t < NT) {
       fill(b ^ 1);
@@ -494,6 +507,7 @@ extern "C" __global__ void __launch_bounds__(NTB) rfx_plan_compact(
     __syncthreads();
     const u64 base = s_prefix;
     const u32 total = s_total[b];
+    if (EARLY && t == NT) s_next = atomicAdd(tile_counter, 1u);
     const u64* st = sstage + (size_t)b * NO * TILE;
     for (u32 r = t; r < total; r += NTB) {
       const u64 pos = base + r;
