@@ -8,6 +8,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <unordered_map>
 #include <mutex>
 #include <utility>
 #include <vector>
@@ -31,6 +32,14 @@ struct Nvrtc {
 std::mutex g_mu;
 Nvrtc g_nv;
 std::map<std::pair<int, std::string>, cudaKernel_t> g_cache;
+struct PlanHash {
+  size_t operator()(const std::pair<int, std::string>& k) const {
+    return std::hash<std::string>()(k.second) ^ ((size_t)k.first << 48);
+  }
+};
+// plan keys seen, to the kernels in g_cache; emptied when it has kMaxPlans
+std::unordered_map<std::pair<int, std::string>, cudaKernel_t, PlanHash> g_plans;
+constexpr size_t kMaxPlans = 4096;
 
 bool env_disabled() {
   const char* e = std::getenv("RFX_JIT");
@@ -108,6 +117,28 @@ rfx_status jit_kernel(const std::string& source, const char* name, cudaKernel_t*
   }
   g_cache[key] = k;
   *out = k;
+  return RFX_OK;
+}
+
+rfx_status jit_plan_kernel(const std::string& key, const std::function<std::string()>& source, const char* name,
+                           cudaKernel_t* out) {
+  if (env_disabled()) return RFX_ERR_UNSUPPORTED;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return RFX_ERR_CUDA;
+  auto k = std::make_pair(dev, key);
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    auto it = g_plans.find(k);
+    if (it != g_plans.end()) {
+      *out = it->second;
+      return RFX_OK;
+    }
+  }
+  const rfx_status st = jit_kernel(source(), name, out);
+  if (st != RFX_OK) return st;
+  std::lock_guard<std::mutex> lk(g_mu);
+  if (g_plans.size() >= kMaxPlans) g_plans.clear();
+  g_plans[std::move(k)] = *out;
   return RFX_OK;
 }
 

@@ -9,6 +9,7 @@
 
 #include <cuda_runtime.h>
 
+#include <functional>
 #include <string>
 
 #include "rfx/rfx.h"
@@ -22,5 +23,11 @@ rfx_status jit_kernel(const std::string& source, const char* name, cudaKernel_t*
 
 // Whether runtime compilation is enabled and NVRTC could be opened.
 bool jit_available();
+
+// jit_kernel for a plan named by `key` (everything its source depends on): the source is only
+// generated when the key is new on this device.  Generating the text took 15 to 20 us, most
+// of the host time of a prepared plan's launch.
+rfx_status jit_plan_kernel(const std::string& key, const std::function<std::string()>& source, const char* name,
+                           cudaKernel_t* out);
 
 }  // namespace rfx

@@ -548,6 +548,15 @@ ScanProgram without_consts(const ScanProgram& p) {
   return q;
 }
 
+// The key of a plan's kernel: the generator's arguments and the program's bytes.
+std::string plan_key(char kind, const ScanProgram& p, uint32_t a, uint32_t b, uint32_t c) {
+  const uint32_t args[3] = {a, b, c};
+  std::string k(1, kind);
+  k.append(reinterpret_cast<const char*>(args), sizeof(args));
+  k.append(reinterpret_cast<const char*>(&p), sizeof(p));   // cleared before it was filled in
+  return k;
+}
+
 }  // namespace
 
 // Launches the specialised aggregate kernel; RFX_ERR_UNSUPPORTED when it cannot be
@@ -563,7 +572,9 @@ rfx_status jit_aggregate(const ScanProgram& p, const void* in, uint64_t n, unsig
   if (variant == 1) rows += 1;
   if (variant == 2 && rows > 1) rows -= 1;
   cudaKernel_t k;
-  rfx_status st = jit_kernel(gen_aggregate(without_consts(p), priv, rows), "rfx_plan_aggregate", &k);
+  const ScanProgram q = without_consts(p);
+  rfx_status st = jit_plan_kernel(plan_key('a', q, priv, (uint32_t)rows, 0),
+                                  [&] { return gen_aggregate(q, priv, rows); }, "rfx_plan_aggregate", &k);
   if (st != RFX_OK) return st;
   const size_t smem = (priv ? (size_t)nacc * kJitThreads : (size_t)nacc) * sizeof(uint64_t);
   RFX_CUDA_TRY(allow_smem((const void*)k, smem));
@@ -590,7 +601,9 @@ rfx_status jit_compact(const ScanProgram& p, int mode, const void* in, uint64_t 
   if ((uint64_t)ipt * kJitThreads < tile_rows) ipt = (int)(tile_rows / kJitThreads);
   tile_rows = (uint64_t)ipt * kJitThreads;
   cudaKernel_t k;
-  rfx_status st = jit_kernel(gen_compact(without_consts(p), mode, wout, ipt), "rfx_plan_compact", &k);
+  const ScanProgram q = without_consts(p);
+  rfx_status st = jit_plan_kernel(plan_key('c', q, (uint32_t)mode, wout, (uint32_t)ipt),
+                                  [&] { return gen_compact(q, mode, wout, ipt); }, "rfx_plan_compact", &k);
   if (st != RFX_OK) return st;
   const uint64_t tiles = (n + tile_rows - 1) / tile_rows;
   const uint32_t no = (wout + 7) / 8;
