@@ -110,3 +110,27 @@ def test_reduce_tuples_variants(cuda, variant, n, distinct):
         R.tune_force(1, -1)
     ek, es, ec = _expect(rows, 96, 0, 64, 4)
     assert np.array_equal(k, ek) and np.array_equal(s, es) and np.array_equal(c, ec)
+
+
+@pytest.mark.parametrize("rb,ks", [(16, 96), (16, 64), (8, 32)])
+@pytest.mark.parametrize("n", [256, 257, 70_001])
+def test_dense_and_clustered_groups(cuda, rb, ks, n):
+    """Groups of one row, of a few, and long runs between clusters of short ones: tiles whose
+    groups are gathered before they are written beside tiles whose lanes write their own, and
+    sub-chunks with more groups than their scratch holds."""
+    rng = np.random.default_rng(n + ks)
+    for kind in range(3):
+        if kind == 0:
+            ids = np.arange(n)
+        elif kind == 1:
+            ids = np.sort(rng.integers(0, n, n))
+        else:
+            ids = np.cumsum((np.arange(n) // 300 % 2 == 0) & (rng.random(n) < 0.7))
+        rows = rng.integers(0, 256, (n, rb), dtype=np.uint8)
+        kbytes = rb - ks // 8
+        for b in range(kbytes):
+            rows[:, ks // 8 + b] = ((ids >> (8 * b)) & 0xff).astype(np.uint8) if b < 4 else 0
+        vbits = 64 if rb == 16 else 32
+        ek, es, ec = _expect(rows, ks, 0, vbits, 4)
+        k, s, c = _run(cuda, rows, ks, 0, vbits, 4)
+        assert np.array_equal(k, ek) and np.array_equal(s, es) and np.array_equal(c, ec)
