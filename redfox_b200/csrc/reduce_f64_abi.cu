@@ -459,6 +459,8 @@ __global__ void __launch_bounds__(256) f64_unit_count(F64Args a, uint64_t units)
   __shared__ bool s_last;
   const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const bool vec = (reinterpret_cast<uintptr_t>(a.keys) & 15u) == 0;
+  grid_wait();   // chained launch
+  grid_release();
   const uint64_t nw = (uint64_t)gridDim.x * 8;
   for (uint64_t u = (uint64_t)blockIdx.x * 8 + warp; u < units; u += nw) {
     const uint64_t e0 = u * a.unit, e1 = min(e0 + (uint64_t)a.unit, a.n);
@@ -516,6 +518,8 @@ __global__ void __launch_bounds__(256) f64_unit_count(F64Args a, uint64_t units)
 
 // The largest biased exponent of the finite values (the 3-limb pass's window).
 __global__ void __launch_bounds__(256) f64_emax(F64Args a) {
+  grid_wait();   // chained launch
+  grid_release();
   if (gated_off(a)) return;
   int m = 1;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -534,6 +538,8 @@ __global__ void __launch_bounds__(256) f64_emax(F64Args a) {
 // step's loads in flight 106, the 3-limb integers 174; MIN 73 / 98 / 90, before 100.
 template <int KB, class Op>
 __global__ void __launch_bounds__(256, Op::BLOCKS) f64_unit_kernel(F64Args a, uint64_t units) {
+  grid_wait();   // chained launch
+  grid_release();
   if (gated_off(a)) return;
   using P = typename Op::P;
   constexpr int V = kF64WarpIPT;
@@ -635,6 +641,8 @@ __global__ void __launch_bounds__(256, Op::BLOCKS) f64_unit_kernel(F64Args a, ui
 // without a head, 32 at a time; every unit is walked over by one warp only.
 template <class Op>
 __global__ void __launch_bounds__(256) f64_fix(F64Args a, uint64_t units) {
+  grid_wait();   // chained launch
+  grid_release();
   if (gated_off(a)) return;
   using P = typename Op::P;
   const uint32_t lane = threadIdx.x & 31;
@@ -748,10 +756,8 @@ template <int KB, class Op>
 rfx_status f64_run_units(const F64Args& a, uint64_t units, cudaStream_t s) {
   const uint64_t want = (units + 7) / 8;
   const int gm = persistent_grid((const void*)f64_unit_kernel<KB, Op>, 256, 0, want);
-  f64_unit_kernel<KB, Op><<<gm, 256, 0, s>>>(a, units);
-  RFX_CUDA_TRY(cudaGetLastError());
-  f64_fix<Op><<<(int)want, 256, 0, s>>>(a, units);
-  RFX_CUDA_TRY(cudaGetLastError());
+  RFX_CUDA_TRY(launch_chained(f64_unit_kernel<KB, Op>, gm, 256, 0, s, a, units));
+  RFX_CUDA_TRY(launch_chained(f64_fix<Op>, (int)want, 256, 0, s, a, units));
   return RFX_OK;
 }
 
@@ -778,8 +784,7 @@ rfx_status f64_dispatch_op(F64Args a, uint32_t op, void* ws, cudaStream_t s) {
   a.inexact = l.inexact_narrow;
   a.emax = l.emax;
   const int ge = persistent_grid((const void*)f64_emax, 256, 0, (a.n + 2047) / 2048);
-  f64_emax<<<ge, 256, 0, s>>>(a);
-  RFX_CUDA_TRY(cudaGetLastError());
+  RFX_CUDA_TRY(launch_chained(f64_emax, ge, 256, 0, s, a));
   st = f64_run_units<KB, SumOp<kNarrowLimbs>>(a, units, s);
   if (st != RFX_OK) return st;
   a.gate = l.inexact_narrow;

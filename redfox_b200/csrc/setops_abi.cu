@@ -125,23 +125,21 @@ rfx_status launch_seg(int mode, SetFilterArgs& a, const FilterLayout& L, cudaStr
     if (!wcap || (a.na && !aligned16(a.a)) || (a.nb && !aligned16(a.b))) return RFX_ERR_UNSUPPORTED;
     if (tiles) {
       const uint64_t work = (tiles + 1) * 32;   // one warp per tile boundary
-      set_bounds_kernel<E, TILE><<<(int)((work + 255) / 256), 256, 0, s>>>(a.a, a.na, a.b, a.nb, L.split);
-      RFX_CUDA_TRY(cudaGetLastError());
+      RFX_CUDA_TRY(launch_chained(set_bounds_kernel<E, TILE>, (int)((work + 255) / 256), 256, 0, s, a.a, a.na, a.b, a.nb,
+                                  L.split));
       a.split = L.split;
       a.wcap = wcap;
       auto k = mode == KEEP_MATCHED ? set_mark_seg_kernel<E, KEEP_MATCHED, IPT> : set_mark_seg_kernel<E, KEEP_UNMATCHED, IPT>;
       const size_t smem = 2 * (size_t)seg_buffer_elems<E>(wcap) * E;
       RFX_CUDA_TRY(allow_smem((const void*)k, smem));
       const int grid = persistent_grid((const void*)k, kSetThreads, smem, tiles);
-      k<<<grid, kSetThreads, smem, s>>>(a, L.mask, L.counts, L.wcounts);
-      RFX_CUDA_TRY(cudaGetLastError());
+      RFX_CUDA_TRY(launch_chained(k, grid, kSetThreads, smem, s, a, L.mask, L.counts, L.wcounts));
     }
-    set_offsets_kernel<<<1, kOffsetThreads, 0, s>>>(L.counts, tiles, L.offsets, a.d_count);
-    RFX_CUDA_TRY(cudaGetLastError());
+    RFX_CUDA_TRY(launch_chained(set_offsets_kernel, 1, kOffsetThreads, 0, s, L.counts, tiles, L.offsets, a.d_count));
     if (tiles) {
       const int grid = persistent_grid((const void*)set_compact_seg_kernel<E, IPT>, kSetThreads, 0, tiles);
-      set_compact_seg_kernel<E, IPT><<<grid, kSetThreads, 0, s>>>(a.a, a.na, L.mask, L.offsets, L.wcounts, a.out, a.na);
-      RFX_CUDA_TRY(cudaGetLastError());
+      RFX_CUDA_TRY(launch_chained(set_compact_seg_kernel<E, IPT>, grid, kSetThreads, 0, s, a.a, a.na, L.mask, L.offsets,
+                                  L.wcounts, a.out, a.na));
     }
     return RFX_OK;
   }
@@ -196,16 +194,13 @@ rfx_status launch_merge(const void* a, uint64_t na, const void* d, uint64_t nd_m
     // the staged merge: partitions of every tile first, then the tiles
     if (mp && aligned16(a) && aligned16(d) && aligned16(out)) {
       const uint64_t work = (tiles + 1) * 32;   // one warp per tile boundary
-      merge_partition_kernel<E><<<(int)((work + 255) / 256), 256, 0, s>>>(
-          static_cast<const uint8_t*>(a), na, static_cast<const uint8_t*>(d), nd_max, d_nd, mp);
-      RFX_CUDA_TRY(cudaGetLastError());
+      RFX_CUDA_TRY(launch_chained(merge_partition_kernel<E>, (int)((work + 255) / 256), 256, 0, s,
+                                  static_cast<const uint8_t*>(a), na, static_cast<const uint8_t*>(d), nd_max, d_nd, mp));
       const size_t smem = merge_staged_smem<E>();
       RFX_CUDA_TRY(allow_smem((const void*)merge_staged_kernel<E>, smem));
       const int grid = persistent_grid((const void*)merge_staged_kernel<E>, kSetThreads, smem, tiles ? tiles : 1);
-      merge_staged_kernel<E><<<grid, kSetThreads, smem, s>>>(static_cast<const uint8_t*>(a), na,
-                                                              static_cast<const uint8_t*>(d), nd_max, d_nd, mp,
-                                                              static_cast<uint8_t*>(out), d_count);
-      RFX_CUDA_TRY(cudaGetLastError());
+      RFX_CUDA_TRY(launch_chained(merge_staged_kernel<E>, grid, kSetThreads, smem, s, static_cast<const uint8_t*>(a), na,
+                                  static_cast<const uint8_t*>(d), nd_max, d_nd, mp, static_cast<uint8_t*>(out), d_count));
       return RFX_OK;
     }
   }

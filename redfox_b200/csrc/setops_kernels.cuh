@@ -351,6 +351,8 @@ constexpr int kOffsetThreads = 1024;
 
 __global__ void __launch_bounds__(kOffsetThreads)
 set_offsets_kernel(const uint32_t* counts, uint64_t tiles, uint64_t* offsets, uint64_t* d_count) {
+  grid_wait();   // chained launch
+  grid_release();
   __shared__ uint64_t s_w[kOffsetThreads / 32];
   __shared__ uint64_t s_carry;
   const uint32_t t = threadIdx.x, lane = t & 31, w = t >> 5;
@@ -476,6 +478,8 @@ constexpr int kSegWarps = kSetThreads / 32;
 // value of tile k lies between its own first element and boundary k + 1's.
 template <int E, int TILE>
 __global__ void set_bounds_kernel(const uint8_t* a, uint64_t na, const uint8_t* b, uint64_t nb, uint64_t* split) {
+  grid_wait();   // chained launch
+  grid_release();
   const KeyView<E> A{a, na, 0};
   const KeyView<E> B{b, nb, 0};
   const uint32_t lane = threadIdx.x & 31;
@@ -530,6 +534,8 @@ __device__ __forceinline__ void load_items_vec(const uint8_t* a, uint64_t first,
 template <int E, int MODE, int IPT>
 __global__ void __launch_bounds__(kSetThreads)
 set_mark_seg_kernel(const SetFilterArgs p, uint8_t* mask, uint32_t* counts, uint32_t* wcounts) {
+  grid_wait();   // chained launch
+  grid_release();
   static_assert(E == 4 || E == 8, "4- and 8-byte elements");
   typedef SetWord<E> WT;
   constexpr int kTile = kSetThreads * IPT;
@@ -701,6 +707,8 @@ template <int E, int IPT>
 __global__ void __launch_bounds__(kSetThreads)
 set_compact_seg_kernel(const uint8_t* a, uint64_t na, const uint8_t* mask, const uint64_t* offsets,
                        const uint32_t* wcounts, uint8_t* out, uint64_t cap) {
+  grid_wait();   // chained launch
+  grid_release();
   static_assert(E == 4 || E == 8, "4- and 8-byte elements");
   typedef SetWord<E> WT;
   constexpr int kTile = kSetThreads * IPT;
@@ -861,6 +869,8 @@ merge_kernel(const uint8_t* a, uint64_t na, const uint8_t* d, uint64_t nd_max, c
 template <int E>
 __global__ void merge_partition_kernel(const uint8_t* a, uint64_t na, const uint8_t* d, uint64_t nd_max,
                                        const uint64_t* d_nd, uint64_t* mp) {
+  grid_wait();   // chained launch
+  grid_release();
   const uint64_t nd = d_nd ? min(nd_max, *d_nd) : nd_max;
   const uint64_t total = na + nd;
   const uint64_t tiles = (total + kMergeTile - 1) / kMergeTile;
@@ -890,6 +900,8 @@ template <int E>
 __global__ void __launch_bounds__(kSetThreads)
 merge_staged_kernel(const uint8_t* a, uint64_t na, const uint8_t* d, uint64_t nd_max, const uint64_t* d_nd,
                     const uint64_t* mp, uint8_t* out, uint64_t* d_count) {
+  grid_wait();   // chained launch
+  grid_release();
   static_assert(E == 4 || E == 8, "4- and 8-byte elements");
   typedef SetWord<E> WT;
   constexpr uint32_t kBuf = merge_buffer_elems<E>();
