@@ -35,12 +35,22 @@ def gen_join_aggregate(nr=C0_R_ROWS, ns=C0_S_ROWS, key_domain=C0_KEY_DOMAIN, dev
     return r, s
 
 
+def _packed(rows):
+    """rows as the sorts read them: contiguous, at an address of 16 bytes' alignment.  The tensor
+    itself where it is so, else a copy (a view of every second row, a view from an odd offset)."""
+    if rows.is_contiguous() and rows.data_ptr() % 16 == 0:
+        return rows
+    import torch
+    return rows.clone(memory_format=torch.contiguous_format)
+
+
 def join_aggregate(r, s, stream=None):
     """sort R, sort S, join on key, SUM(amount) and COUNT by key.
     Returns (keys u32, sums int64, counts u32, join_rows)."""
-    r, _ = R.sorted_copy(r, begin_bit=32, end_bit=64, stream=stream)     # R on its key field
-    s, _ = R.sorted_copy(s, begin_bit=64, end_bit=96, stream=stream)     # S on its key field
-    out, total = R.join_tuples_two_step(r, 32, s, 64, 16, stream=stream)   # (key, payload, amount)
+    r, s = _packed(r), _packed(s)   # held until the end: the sorts read them in stream order
+    rs, _ = R.sorted_copy(r, begin_bit=32, end_bit=64, stream=stream)    # R on its key field
+    ss, _ = R.sorted_copy(s, begin_bit=64, end_bit=96, stream=stream)    # S on its key field
+    out, total = R.join_tuples_two_step(rs, 32, ss, 64, 16, stream=stream)   # (key, payload, amount)
     keys, sums, counts, g = R.reduce_tuples(out, 96, 0, 64, 4, n=total, stream=stream)
     return keys, sums, counts, total
 
@@ -118,6 +128,7 @@ def three_relation(d1, d2, f, list_in, list_out, f_sorted=None, stream=None):
     keys = R.set_op(R.SET_INTERSECTION, keys, list_in, stream=stream)
     keys = R.set_op(R.SET_DIFFERENCE, keys, list_out, stream=stream)
     if f_sorted is None:
+        f = _packed(f)   # held until the end: the sort reads it in stream order
         f_sorted, _ = R.sorted_copy(f, begin_bit=64, end_bit=96, stream=stream)       # on fk
     keys4 = keys.view(torch.uint8).view(-1, 4)
     j2, total = R.join_tuples_two_step(keys4, 0, f_sorted, 64, 16, stream=stream)     # (pk2, amount)
