@@ -682,6 +682,8 @@ __global__ void __launch_bounds__(256) f64_fix(F64Args a, uint64_t units) {
   if (!head && !last) return;
   const P* first_of = reinterpret_cast<const P*>(a.first);
   const P* last_of = reinterpret_cast<const P*>(a.last);
+  // an addition that lost bits counts in whichever lane it was made, but only where the sum
+  // goes into the run: lanes beyond the stop hold units of earlier runs
   bool bad = false;
   P acc = Op::identity();
   // 32 units at first (the last head is usually near), then R consecutive ones per lane
@@ -690,7 +692,7 @@ __global__ void __launch_bounds__(256) f64_fix(F64Args a, uint64_t units) {
   for (int r = 1; pos >= 0; r = R) {
     // this lane's units, the newest first, up to one with a head
     P x = Op::identity();
-    bool h = false;
+    bool h = false, lost = false;
     if (r == 1) {
       const int64_t v = pos - lane;
       if (v >= 0) {
@@ -706,19 +708,22 @@ __global__ void __launch_bounds__(256) f64_fix(F64Args a, uint64_t units) {
         const bool hk = a.heads[c] > 0;
         const P y = hk ? last_of[c] : first_of[c];
         if (v >= 0 && !h) {
-          x = Op::combine(y, x, bad);
+          x = Op::combine(y, x, lost);
           h = hk;
         }
       }
     }
     const uint32_t m = __ballot_sync(0xffffffffu, h);
     const uint32_t stop = m ? __ffs(m) - 1 : 31u;   // the nearest lane with a head
-    if (lane > stop) x = Op::identity();
-    // in order: a higher lane holds earlier units
+    if (lane > stop)
+      x = Op::identity();
+    else
+      bad = bad || lost;
+    // in order: a higher lane holds earlier units; the lanes that lead to lane 0
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const P y = shfl_down_any(x, o);
-      if (lane + o < 32) x = Op::combine(y, x, bad);
+      if ((lane & (2 * o - 1)) == 0) x = Op::combine(y, x, bad);
     }
     acc = Op::combine(shfl_any(x, 0), acc, bad);
     if (m) break;
@@ -732,8 +737,8 @@ __global__ void __launch_bounds__(256) f64_fix(F64Args a, uint64_t units) {
     }
     if (last && head)
       a.out_vals[base + a.heads[u] - 1] = __longlong_as_double((long long)Op::finalize(last_of[u], L));
-    if (bad) atomicOr(a.inexact, 1u);
   }
+  if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.inexact, 1u);
 }
 
 // ------------------------------------------------------------------ scalar reductions

@@ -247,3 +247,35 @@ def test_sum_pair_signs_and_cancellation(cuda):
                     np.float64)
     keys = np.array([0, 0, 1, 1, 2, 2, 2, 3, 3, 3, 4, 4, 5, 5], np.uint32)
     _check_sum(cuda, keys, vals)
+
+
+def _one_run_sum(cuda, vals):
+    """The column's sum as one run, and the exactly rounded one."""
+    _, ov, g = R.reduce_f64(None, _dev(vals, cuda), R.F64_SUM)
+    assert g == 1
+    return to_np(ov), np.array([O.exact_sum(vals)])
+
+
+@pytest.mark.parametrize("units", [4, 6, 31, 40, 300, 700])
+def test_sum_loss_between_units(cuda, units):
+    """A run over several 256-element units whose only inexact addition joins the sums of two
+    units: 1 + 2^-53 in one and 2^-200 in the next, wherever they lie before the run's end."""
+    n = 256 * units
+    places = sorted({*range(min(units - 1, 36)), units // 2, *range(max(0, units - 36), units - 1)})
+    for p in places:
+        vals = np.zeros(n)
+        vals[256 * p], vals[256 * p + 1], vals[256 * (p + 1)] = 1.0, 2.0**-53, 2.0**-200
+        got, exact = _one_run_sum(cuda, vals)
+        assert exact[0] == 1.0 + 2.0**-52 and _same_bits(got, exact), p
+
+
+def test_sum_loss_that_cancels_later(cuda):
+    """Units that cancel but for what was lost among them, in a run of its own and with more
+    runs after it."""
+    vals = np.zeros(6 * 256)
+    vals[[256, 257, 512, 768, 1024]] = 1e16, 1.0, 1e-17, -1e16, -1.0
+    got, exact = _one_run_sum(cuda, vals)
+    assert exact[0] == 1e-17 and _same_bits(got, exact)
+    keys = np.repeat(np.array([7, 9, 11], np.uint32), [5 * 256, 100, 156])
+    _, ov, g = R.reduce_f64(_dev(keys, cuda), _dev(vals, cuda), R.F64_SUM)
+    assert g == 3 and _same_bits(to_np(ov), O.reduce_f64_exact(keys, vals)[1])
