@@ -239,8 +239,9 @@ struct PairOp {
     const double s = two_sum(a.hi, b.hi, e);
     const double l = two_sum(a.lo, b.lo, e2);
     const double t = two_sum(l, e, e3);
-    bad = bad || !(e2 == 0.0) || !(e3 == 0.0);
     const double h = two_sum(s, t, r);   // keeps the low part below the high one's last place
+    // (r is not finite after an overflow of that last addition alone)
+    bad = bad || !(e2 == 0.0) || !(e3 == 0.0) || !isfinite(r);
     return t == 0.0 ? P{s, 0.0} : P{h, r};   // (s + 0 would lose the sign of a zero)
   }
   __device__ __forceinline__ static unsigned long long finalize(const P& p, int) {

@@ -279,3 +279,22 @@ def test_sum_loss_that_cancels_later(cuda):
     keys = np.repeat(np.array([7, 9, 11], np.uint32), [5 * 256, 100, 156])
     _, ov, g = R.reduce_f64(_dev(keys, cuda), _dev(vals, cuda), R.F64_SUM)
     assert g == 3 and _same_bits(to_np(ov), O.reduce_f64_exact(keys, vals)[1])
+
+
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+@pytest.mark.parametrize("terms", [(1, 2, 2), (2, 1, 2), (2, 2, 1)])
+def test_sum_overflows_between_partials(cuda, sign, terms):
+    """The largest double and twice a quarter of its last place: every pair of them stays
+    finite, the sum rounds to infinity.  The run lies across the 8 elements of a lane, a step's
+    256 and a unit's, in every way."""
+    x = {1: np.finfo(np.float64).max, 2: 2.0**969}
+    for at in [*range(0, 18), *range(247, 260), *range(503, 516)]:
+        vals = np.ones(600)
+        vals[at:at + 3] = [sign * x[t] for t in terms]
+        keys = np.zeros(600, np.uint32)
+        keys[at:] = 1
+        keys[at + 3:] = 2
+        ok, ov, g = R.reduce_f64(_dev(keys, cuda), _dev(vals, cuda), R.F64_SUM)
+        ek, es = O.reduce_f64_exact(keys, vals)
+        assert g == es.shape[0] and sign * np.inf in es
+        assert _same_bits(to_np(ov), es), at
