@@ -8,8 +8,8 @@
 //     addition goes to the low part, and an error of the low addition raises a flag.  While
 //     the flag stays down hi + lo is the exact sum whatever the order of the additions, and
 //     one rounding of hi + lo finishes it.  This holds for values whose bits span about 100
-//     binary places, such as amounts of money.
-//   * If the flag went up (a wider span, an overflow, an infinity or a NaN), a second pass
+//     binary places, such as amounts of money, with or without infinities and NaNs.
+//   * If the flag went up (a wider span, a finite value from 2^1000 on), a second pass
 //     works in integers: every double is a 53-bit integer times a power of two, so a run's
 //     sum is accumulated as a two's-complement integer in units of 2^L over W 64-bit limbs
 //     (add with carry).  W = 3 limbs with L set from the largest exponent in the input: exact
@@ -52,6 +52,7 @@ enum : uint32_t { kSumNaN = 1, kSumPosInf = 2, kSumNegInf = 4, kSumNotNegZero = 
 // choice of L, so the result is exact and independent of the order of the additions.
 template <int W>
 struct SumOp {
+  static constexpr bool SCREENS = false;
   static constexpr bool COMMUTES = W == 3;   // (the 34 limbs are not worth another copy)
   static constexpr int BLOCKS = W == 3 ? 2 : 1;   // of 256 threads per SM: the limbs live in registers
   struct P {
@@ -213,38 +214,48 @@ struct SumOp {
 };
 
 // ------------------------------------------------------------------ exact sum in two doubles
-// The sum is hi + lo exactly as long as no flag (`bad`) went up.
+// The sum is hi + lo exactly as long as no flag (`bad`) went up.  Finite values from 2^1000 on
+// raise it by themselves: no sum of 2^30 smaller ones overflows, so a high part that is not
+// finite comes from an infinity or a NaN among the terms, and is what IEEE addition makes of
+// them.  The errors are NaN from there on and say nothing.
 struct PairOp {
   static constexpr int BLOCKS = 4;
+  static constexpr bool SCREENS = true;
   static constexpr bool COMMUTES = true;
   struct P {
     double hi, lo;
   };
   __device__ __forceinline__ static P identity() { return P{-0.0, 0.0}; }   // -0 + x is x for every x
-  // a + b = s + e exactly (Knuth's TwoSum); e is NaN after an overflow or a special.
+  // a + b = s + e exactly (Knuth's TwoSum) when s is finite.
   __device__ __forceinline__ static double two_sum(double a, double b, double& e) {
     const double s = __dadd_rn(a, b);
     const double bb = __dadd_rn(s, -a);
     e = __dadd_rn(__dadd_rn(a, -__dadd_rn(s, -bb)), __dadd_rn(b, -bb));
     return s;
   }
+  __device__ __forceinline__ static bool lost(double e) { return fabs(e) > 0.0; }   // not for a NaN
+  // Twice the high word without the sign, infinities and NaNs wrapped round to the low end.
+  __device__ __forceinline__ static bool large(double x) {
+    constexpr uint32_t kFrom = ((1000u + 1023u) << 21) + (1u << 21);
+    return ((uint32_t)__double2hiint(x) << 1) + (1u << 21) >= kFrom;
+  }
   __device__ __forceinline__ static void add(P& p, double x, int, uint32_t*, bool& bad) {
     double e, e2;
     p.hi = two_sum(p.hi, x, e);
     p.lo = two_sum(p.lo, e, e2);
-    bad = bad || !(e2 == 0.0);   // a NaN is not zero
+    bad = bad || lost(e2);
   }
   __device__ __forceinline__ static P combine(const P& a, const P& b, bool& bad) {
     double e, e2, e3, r;
     const double s = two_sum(a.hi, b.hi, e);
     const double l = two_sum(a.lo, b.lo, e2);
     const double t = two_sum(l, e, e3);
+    bad = bad || lost(e2) || lost(e3);
     const double h = two_sum(s, t, r);   // keeps the low part below the high one's last place
-    // (r is not finite after an overflow of that last addition alone)
-    bad = bad || !(e2 == 0.0) || !(e3 == 0.0) || !isfinite(r);
-    return t == 0.0 ? P{s, 0.0} : P{h, r};   // (s + 0 would lose the sign of a zero)
+    return fabs(t) > 0.0 ? P{h, r} : P{s, 0.0};   // (s + 0 would lose the sign of a zero)
   }
   __device__ __forceinline__ static unsigned long long finalize(const P& p, int) {
+    if (!isfinite(p.hi)) return p.hi != p.hi ? 0x7ff8000000000000ull : (unsigned long long)__double_as_longlong(p.hi);
     return (unsigned long long)__double_as_longlong(p.lo == 0.0 ? p.hi : __dadd_rn(p.hi, p.lo));
   }
 };
@@ -252,6 +263,7 @@ struct PairOp {
 // ------------------------------------------------------------------ minimum (the fold)
 struct MinOp {
   static constexpr int BLOCKS = 4;
+  static constexpr bool SCREENS = false;
   static constexpr bool COMMUTES = false;
   struct P {
     unsigned long long v;  // bits of the fold value (a NaN while pending)
@@ -294,7 +306,7 @@ struct Key {
 };
 
 template <int KB>
-__device__ __forceinline__ Key load_key(const uint8_t* keys, uint64_t i) {
+__device__ __forceinline__ Key load_key(const uint8_t* keys, uint32_t i) {
   if constexpr (KB == 0) return Key{0ull, 0ull};
   if constexpr (KB == 1) return Key{keys[i], 0ull};
   if constexpr (KB == 2) return Key{reinterpret_cast<const uint16_t*>(keys)[i], 0ull};
@@ -308,7 +320,7 @@ __device__ __forceinline__ Key load_key(const uint8_t* keys, uint64_t i) {
 }
 
 template <int KB>
-__device__ __forceinline__ void store_key(uint8_t* out, uint64_t r, const Key& k) {
+__device__ __forceinline__ void store_key(uint8_t* out, uint32_t r, const Key& k) {
   if constexpr (KB == 1) out[r] = (uint8_t)k.lo;
   if constexpr (KB == 2) reinterpret_cast<uint16_t*>(out)[r] = (uint16_t)k.lo;
   if constexpr (KB == 4) reinterpret_cast<uint32_t*>(out)[r] = (uint32_t)k.lo;
@@ -389,8 +401,8 @@ constexpr int kF64UnitMost = 4096;
 
 // Eight consecutive keys from element `first` (a multiple of 8) of a 16-byte aligned array.
 template <int KB>
-__device__ __forceinline__ void load_keys8(const uint8_t* keys, uint64_t first, Key (&k)[8]) {
-  const uint8_t* p = keys + first * KB;
+__device__ __forceinline__ void load_keys8(const uint8_t* keys, uint32_t first, Key (&k)[8]) {
+  const uint8_t* p = keys + (size_t)first * KB;
   if constexpr (KB == 1) {
     const uint2 v = *reinterpret_cast<const uint2*>(p);
 #pragma unroll
@@ -423,7 +435,7 @@ __device__ __forceinline__ void load_keys8(const uint8_t* keys, uint64_t first, 
 
 // Keys first .. first + 7 of the elements before `end`; vec: the array is 16-byte aligned.
 template <int KB>
-__device__ __forceinline__ void load_keys(const uint8_t* keys, uint64_t first, uint64_t end, bool vec, Key (&k)[8]) {
+__device__ __forceinline__ void load_keys(const uint8_t* keys, uint32_t first, uint32_t end, bool vec, Key (&k)[8]) {
   if constexpr (KB == 0) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) k[j] = Key{0ull, 0ull};
@@ -437,7 +449,7 @@ __device__ __forceinline__ void load_keys(const uint8_t* keys, uint64_t first, u
 
 // The heads among a lane's keys (bit j: element first + j starts a run).
 template <int KB>
-__device__ __forceinline__ uint32_t head_bits(const F64Args& a, const Key (&k)[8], uint64_t first, uint64_t end) {
+__device__ __forceinline__ uint32_t head_bits(const F64Args& a, const Key (&k)[8], uint32_t first, uint32_t end) {
   uint32_t hm = first == 0 && end > 0 ? 1u : 0u;
   if constexpr (KB > 0) {
     const uint32_t lane = threadIdx.x & 31;
@@ -467,11 +479,11 @@ __global__ void __launch_bounds__(256) f64_unit_count(F64Args a, uint64_t units)
   grid_release();
   const uint64_t nw = (uint64_t)gridDim.x * 8;
   for (uint64_t u = (uint64_t)blockIdx.x * 8 + warp; u < units; u += nw) {
-    const uint64_t e0 = u * a.unit, e1 = min(e0 + (uint64_t)a.unit, a.n);
+    const uint32_t e0 = (uint32_t)u * a.unit, e1 = min(e0 + a.unit, (uint32_t)a.n);
     uint32_t c = 0;
 #pragma unroll 4
-    for (uint64_t tb = e0; tb < e1; tb += kF64Step) {
-      const uint64_t first = tb + 8ull * lane;
+    for (uint32_t tb = e0; tb < e1; tb += kF64Step) {
+      const uint32_t first = tb + 8 * lane;
       Key k[8];
       load_keys<KB>(a.keys, first, e1, vec, k);
       c += (uint32_t)__popc(head_bits<KB>(a, k, first, e1));
@@ -548,15 +560,15 @@ __global__ void __launch_bounds__(256, Op::BLOCKS) f64_unit_kernel(F64Args a, ui
   using P = typename Op::P;
   constexpr int V = kF64WarpIPT;
   const uint32_t lane = threadIdx.x & 31;
-  const uint64_t gw = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  const uint32_t gw = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const uint32_t nw = gridDim.x * 8;
   const int L = window_L(a);
   const bool vk = (reinterpret_cast<uintptr_t>(a.keys) & 15u) == 0;
   const bool vv = (reinterpret_cast<uintptr_t>(a.vals) & 15u) == 0;
   bool bad = false;
-  for (uint64_t u = gw; u < units; u += nw) {
-    const uint64_t e0 = u * a.unit, e1 = min(e0 + (uint64_t)a.unit, a.n);
-    uint64_t run_base = a.base[u];   // index of the next head's run
+  for (uint32_t u = gw; u < units; u += nw) {
+    const uint32_t e0 = u * a.unit, e1 = min(e0 + a.unit, (uint32_t)a.n);   // below 2^30
+    uint32_t run_base = a.base[u];   // index of the next head's run
     P carry = Op::identity();
     bool carry_head = false;
     // sums of steps without a head stay in their lanes until a head or the unit's end comes
@@ -574,8 +586,8 @@ __global__ void __launch_bounds__(256, Op::BLOCKS) f64_unit_kernel(F64Args a, ui
         holding = false;
       }
     };
-    for (uint64_t tb = e0; tb < e1; tb += kF64Step) {
-      const uint64_t first = tb + (uint64_t)lane * V;
+    for (uint32_t tb = e0; tb < e1; tb += kF64Step) {
+      const uint32_t first = tb + lane * V;
       Key keys[V];
       double vals[V];
       load_keys<KB>(a.keys, first, e1, vk, keys);
@@ -589,6 +601,10 @@ __global__ void __launch_bounds__(256, Op::BLOCKS) f64_unit_kernel(F64Args a, ui
       } else {
 #pragma unroll
         for (int j = 0; j < V; ++j) vals[j] = first + j < e1 ? a.vals[first + j] : 0.0;
+      }
+      if constexpr (Op::SCREENS) {
+#pragma unroll
+        for (int j = 0; j < V; ++j) bad = bad || Op::large(vals[j]);
       }
       const uint32_t hm = head_bits<KB>(a, keys, first, e1);
       if (Op::COMMUTES && !__any_sync(0xffffffffu, hm != 0)) {
@@ -607,10 +623,10 @@ __global__ void __launch_bounds__(256, Op::BLOCKS) f64_unit_kernel(F64Args a, ui
         const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
         if (lane >= (uint32_t)o) inc += y;
       }
-      const uint64_t lane_run = run_base + inc - cnt;
+      const uint32_t lane_run = run_base + inc - cnt;
       // keys at heads; runs that end inside this lane
       P cur = Op::identity(), pfirst = Op::identity();
-      uint64_t r = lane_run;
+      uint32_t r = lane_run;
 #pragma unroll
       for (int j = 0; j < V; ++j) {
         if (first + j < e1) {

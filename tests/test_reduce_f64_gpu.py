@@ -298,3 +298,22 @@ def test_sum_overflows_between_partials(cuda, sign, terms):
         ek, es = O.reduce_f64_exact(keys, vals)
         assert g == es.shape[0] and sign * np.inf in es
         assert _same_bits(to_np(ov), es), at
+
+
+@pytest.mark.parametrize("specials", [(np.inf,), (-np.inf,), (np.nan,), (np.inf, -np.inf), (np.inf, np.inf),
+                                      (2.0**1000,), (2.0**999, -2.0**999), (np.inf, 2.0**1000), (2.0**1023, 2.0**1023)])
+@pytest.mark.parametrize("apart", [1, 8, 256])
+def test_sum_few_specials(cuda, specials, apart):
+    """One or two infinities, NaNs or very large values in a column of amounts, in one lane's
+    elements, across lanes and across units, in runs of a few elements, of a unit and of all:
+    their runs' sums follow IEEE addition, the other runs' are exact."""
+    n = 1500
+    for at in (0, 7, 255, 511, 700, n - 1 - apart):
+        vals = gen_values("prices", n, at)
+        for i, x in enumerate(specials):
+            vals[at + i * apart] = x
+        for groups in (1, 6, 400):
+            keys = gen_keys(4, n, groups, 3)
+            ok, ov, g = R.reduce_f64(_dev(keys, cuda), _dev(vals, cuda), R.F64_SUM)
+            ek, es = O.reduce_f64_exact(keys, vals)
+            assert g == es.shape[0] and np.array_equal(to_np(ok), ek) and _same_bits(to_np(ov), es), (at, groups)
