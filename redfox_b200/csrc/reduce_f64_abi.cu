@@ -52,7 +52,7 @@ enum : uint32_t { kSumNaN = 1, kSumPosInf = 2, kSumNegInf = 4, kSumNotNegZero = 
 // choice of L, so the result is exact and independent of the order of the additions.
 template <int W>
 struct SumOp {
-  static constexpr bool SCREENS = false;
+  static constexpr bool TENTATIVE = false;
   static constexpr bool COMMUTES = W == 3;   // (the 34 limbs are not worth another copy)
   static constexpr int BLOCKS = W == 3 ? 2 : 1;   // of 256 threads per SM: the limbs live in registers
   struct P {
@@ -220,7 +220,7 @@ struct SumOp {
 // them.  The errors are NaN from there on and say nothing.
 struct PairOp {
   static constexpr int BLOCKS = 4;
-  static constexpr bool SCREENS = true;
+  static constexpr bool TENTATIVE = true;   // the pass gives up once a flag is up
   static constexpr bool COMMUTES = true;
   struct P {
     double hi, lo;
@@ -263,7 +263,7 @@ struct PairOp {
 // ------------------------------------------------------------------ minimum (the fold)
 struct MinOp {
   static constexpr int BLOCKS = 4;
-  static constexpr bool SCREENS = false;
+  static constexpr bool TENTATIVE = false;
   static constexpr bool COMMUTES = false;
   struct P {
     unsigned long long v;  // bits of the fold value (a NaN while pending)
@@ -538,10 +538,27 @@ __global__ void __launch_bounds__(256) f64_emax(F64Args a) {
   grid_release();
   if (gated_off(a)) return;
   int m = 1;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += (uint64_t)gridDim.x * blockDim.x) {
-    const int eb = (int)(((unsigned long long)__double_as_longlong(a.vals[i]) >> 52) & 0x7ffu);
+  auto take = [&](double x) {
+    const int eb = (__double2hiint(x) >> 20) & 0x7ff;
     if (eb != 0x7ff && eb > m) m = eb;
+  };
+  // 16 bytes per load, four loads in flight
+  const uint32_t tid = blockIdx.x * 256 + threadIdx.x, stride = gridDim.x * 256, n = (uint32_t)a.n;
+  const uint32_t pairs = (reinterpret_cast<uintptr_t>(a.vals) & 15u) == 0 ? n / 2 : 0u;
+  for (uint32_t c = tid; c < pairs; c += 4 * stride) {
+    double2 v[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+      const uint32_t i = c + k * stride;
+      v[k] = i < pairs ? reinterpret_cast<const double2*>(a.vals)[i] : make_double2(0.0, 0.0);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      take(v[k].x);
+      take(v[k].y);
+    }
   }
+  for (uint32_t i = 2 * pairs + tid; i < n; i += stride) take(a.vals[i]);
   m = __reduce_max_sync(0xffffffffu, m);
   if ((threadIdx.x & 31) == 0) atomicMax(a.emax, m);
 }
@@ -550,8 +567,10 @@ __global__ void __launch_bounds__(256) f64_emax(F64Args a) {
 // (16-byte loads).  A lane folds its elements, writing the runs that start and end among
 // them; a segmented warp scan gives every lane what is open before it.  Bound by the latency
 // of a step's chain (loads, fold, scan), so by the warps resident: 19.3M elements, 256K runs,
-// SUM with 32 warps per SM (64 registers) 87 us, with 24 warps 105, with 16 warps and the next
-// step's loads in flight 106, the 3-limb integers 174; MIN 73 / 98 / 90, before 100.
+// SUM with 32 warps per SM (64 registers, 16 bytes of spills) 85 us, with 24 warps 105, with 16
+// warps and the next step's loads in flight 106, the 3-limb integers 152; MIN 73 / 98 / 90,
+// before 100.  A column that the pair cannot hold is found out in the first steps and costs the
+// pair's pass 15 us (values over 80 binary places), one such value in the middle 30.
 template <int KB, class Op>
 __global__ void __launch_bounds__(256, Op::BLOCKS) f64_unit_kernel(F64Args a, uint64_t units) {
   grid_wait();   // chained launch
@@ -586,7 +605,17 @@ __global__ void __launch_bounds__(256, Op::BLOCKS) f64_unit_kernel(F64Args a, ui
         holding = false;
       }
     };
+    uint32_t raised = 0;
     for (uint32_t tb = e0; tb < e1; tb += kF64Step) {
+      if constexpr (Op::TENTATIVE) {
+        // this pass is for nothing once a flag is up: this warp's, or another's, looked at
+        // every fourth step
+        if (__any_sync(0xffffffffu, bad || raised)) {
+          if (lane == 0) atomicOr(a.inexact, 1u);
+          return;
+        }
+        if ((tb / kF64Step & 3) == 3) raised = ld_relaxed_u32(a.inexact);
+      }
       const uint32_t first = tb + lane * V;
       Key keys[V];
       double vals[V];
@@ -602,7 +631,7 @@ __global__ void __launch_bounds__(256, Op::BLOCKS) f64_unit_kernel(F64Args a, ui
 #pragma unroll
         for (int j = 0; j < V; ++j) vals[j] = first + j < e1 ? a.vals[first + j] : 0.0;
       }
-      if constexpr (Op::SCREENS) {
+      if constexpr (Op::TENTATIVE) {
 #pragma unroll
         for (int j = 0; j < V; ++j) bad = bad || Op::large(vals[j]);
       }
@@ -694,6 +723,7 @@ __global__ void __launch_bounds__(256) f64_fix(F64Args a, uint64_t units) {
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t u = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (u >= units) return;
+  if (Op::TENTATIVE && __any_sync(0xffffffffu, ld_relaxed_u32(a.inexact))) return;
   const int L = window_L(a);
   const bool head = a.heads[u] > 0, last = u == units - 1;
   if (!head && !last) return;

@@ -317,3 +317,16 @@ def test_sum_few_specials(cuda, specials, apart):
             ok, ov, g = R.reduce_f64(_dev(keys, cuda), _dev(vals, cuda), R.F64_SUM)
             ek, es = O.reduce_f64_exact(keys, vals)
             assert g == es.shape[0] and np.array_equal(to_np(ok), ek) and _same_bits(to_np(ov), es), (at, groups)
+
+
+@pytest.mark.parametrize("at", [0, 3 * 1280 + 255, 2_000_000, 4_800_000])
+def test_sum_one_value_outside_the_pair(cuda, at):
+    """Units of five steps, one value that the pair of doubles cannot hold beside the others:
+    units that have ended, that stop at the flag and that never see it."""
+    n = 4737 * 256 * 4
+    vals = gen_values("prices", n, 5)
+    vals[at] = 1e-15
+    keys = gen_keys(4, n, 1000, 6)
+    ok, ov, g = R.reduce_f64(_dev(keys, cuda), _dev(vals, cuda), R.F64_SUM)
+    ek, es = O.reduce_f64_exact(keys, vals)
+    assert g == es.shape[0] and np.array_equal(to_np(ok), ek) and _same_bits(to_np(ov), es)
