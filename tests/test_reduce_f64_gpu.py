@@ -330,3 +330,26 @@ def test_sum_one_value_outside_the_pair(cuda, at):
     ok, ov, g = R.reduce_f64(_dev(keys, cuda), _dev(vals, cuda), R.F64_SUM)
     ek, es = O.reduce_f64_exact(keys, vals)
     assert g == es.shape[0] and np.array_equal(to_np(ok), ek) and _same_bits(to_np(ov), es)
+
+
+@pytest.mark.parametrize("units", [33, 34, 40, 289, 290, 297, 4385, 4386, 4400, 4700])
+@pytest.mark.parametrize("kind", ["prices", "wide", "min"])
+def test_runs_over_many_units(cuda, kind, units):
+    """A run that ends a few units before the last one, from its first unit to its last: looked
+    back over by a warp (32 units), by a block's threads (256 more) and by 4096 at a time, with
+    another block's run before it.  Values whose sum, and whose fold, depends on every one."""
+    n = 256 * units
+    rng = np.random.default_rng(units)
+    vals = gen_values("wide" if kind == "wide" else "prices", n, units)
+    for lead, tail in ((0, 0), (1, 0), (700, 1), (256 * 5, 256 * 3 + 7)):
+        keys = np.full(n, 5, np.uint32)
+        keys[:lead], keys[n - tail:] = np.arange(lead), 9
+        if kind == "min":
+            vals[rng.integers(lead, n - tail)] = -vals[lead]
+            vals[max(0, n - tail - 1)] = np.nan if units % 2 else -1e9
+            ok, ov, g = R.reduce_f64(_dev(keys, cuda), _dev(vals, cuda), R.F64_MIN)
+            ek, es = O.reduce_f64_seq(keys, vals, op_min=True)
+        else:
+            ok, ov, g = R.reduce_f64(_dev(keys, cuda), _dev(vals, cuda), R.F64_SUM)
+            ek, es = O.reduce_f64_exact(keys, vals)
+        assert g == es.shape[0] and np.array_equal(to_np(ok), ek) and _same_bits(to_np(ov), es), (lead, tail)
