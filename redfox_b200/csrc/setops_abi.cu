@@ -191,16 +191,21 @@ rfx_status launch_merge(const void* a, uint64_t na, const void* d, uint64_t nd_m
                         uint64_t* d_count, uint64_t* mp, cudaStream_t s) {
   const uint64_t tiles = (na + nd_max + kMergeTile - 1) / kMergeTile;
   if constexpr (E == 4 || E == 8) {
-    // the staged merge: partitions of every tile first, then the tiles
+    // the staged merge: partitions of every tile first, then the tiles.  Launched plainly, unlike
+    // the filters' kernels: chained, the partition's searches ran beside blocks that already
+    // waited, 40 us instead of 27 for 30M + 12M u32 (the whole union 291 -> 276, 281 before).
     if (mp && aligned16(a) && aligned16(d) && aligned16(out)) {
       const uint64_t work = (tiles + 1) * 32;   // one warp per tile boundary
-      RFX_CUDA_TRY(launch_chained(merge_partition_kernel<E>, (int)((work + 255) / 256), 256, 0, s,
-                                  static_cast<const uint8_t*>(a), na, static_cast<const uint8_t*>(d), nd_max, d_nd, mp));
+      merge_partition_kernel<E><<<(int)((work + 255) / 256), 256, 0, s>>>(
+          static_cast<const uint8_t*>(a), na, static_cast<const uint8_t*>(d), nd_max, d_nd, mp);
+      RFX_CUDA_TRY(cudaGetLastError());
       const size_t smem = merge_staged_smem<E>();
       RFX_CUDA_TRY(allow_smem((const void*)merge_staged_kernel<E>, smem));
       const int grid = persistent_grid((const void*)merge_staged_kernel<E>, kSetThreads, smem, tiles ? tiles : 1);
-      RFX_CUDA_TRY(launch_chained(merge_staged_kernel<E>, grid, kSetThreads, smem, s, static_cast<const uint8_t*>(a), na,
-                                  static_cast<const uint8_t*>(d), nd_max, d_nd, mp, static_cast<uint8_t*>(out), d_count));
+      merge_staged_kernel<E><<<grid, kSetThreads, smem, s>>>(static_cast<const uint8_t*>(a), na,
+                                                              static_cast<const uint8_t*>(d), nd_max, d_nd, mp,
+                                                              static_cast<uint8_t*>(out), d_count);
+      RFX_CUDA_TRY(cudaGetLastError());
       return RFX_OK;
     }
   }

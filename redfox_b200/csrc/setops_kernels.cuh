@@ -869,8 +869,6 @@ merge_kernel(const uint8_t* a, uint64_t na, const uint8_t* d, uint64_t nd_max, c
 template <int E>
 __global__ void merge_partition_kernel(const uint8_t* a, uint64_t na, const uint8_t* d, uint64_t nd_max,
                                        const uint64_t* d_nd, uint64_t* mp) {
-  grid_wait();   // chained launch
-  grid_release();
   const uint64_t nd = d_nd ? min(nd_max, *d_nd) : nd_max;
   const uint64_t total = na + nd;
   const uint64_t tiles = (total + kMergeTile - 1) / kMergeTile;
@@ -900,8 +898,6 @@ template <int E>
 __global__ void __launch_bounds__(kSetThreads)
 merge_staged_kernel(const uint8_t* a, uint64_t na, const uint8_t* d, uint64_t nd_max, const uint64_t* d_nd,
                     const uint64_t* mp, uint8_t* out, uint64_t* d_count) {
-  grid_wait();   // chained launch
-  grid_release();
   static_assert(E == 4 || E == 8, "4- and 8-byte elements");
   typedef SetWord<E> WT;
   constexpr uint32_t kBuf = merge_buffer_elems<E>();
