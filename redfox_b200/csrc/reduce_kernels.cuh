@@ -930,7 +930,7 @@ __device__ __forceinline__ SegPair shfl_seg(const SegPair& x, uint32_t src) {
                  __shfl_sync(0xffffffffu, x.h, src)};
 }
 
-constexpr uint32_t kGatherEnds = 4;   // run heads in one lane from which a tile's groups are gathered
+constexpr uint32_t kGatherEnds = 4;   // run heads in one lane from which the next tile's groups are gathered
 
 template <int RB, int SHAPE, int S, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 2) reduce_warps_kernel(const __grid_constant__ CUtensorMap map,
@@ -982,10 +982,12 @@ __global__ void __launch_bounds__(WARPS * 32, 2) reduce_warps_kernel(const __gri
   Key first_key = 0;
   uint32_t max_lf = 0;
   // 4-byte output keys: a group is 16 bytes, and a tile's groups (one per row at the most) fit
-  // the stage its rows came in.  A tile in which some lane has several is gathered there and
-  // written in order; else each lane writes its own, one round per group of the lane with the
-  // most, which lets the stage be refilled sooner.  38M rows of 16 bytes, us, written by lane / gathered: 75 rows per group 134 / 144,
-  // 10 224 / 248, 4 390 / 387, 3 392 / 352, 2 467 / 360, 1 615 / 373.
+  // the stage its rows came in.  After a tile in which some lane held several, a tile's groups
+  // are gathered there and written in order; else each lane writes its own, one round per group
+  // of the lane with the most, and the stage is refilled as soon as the rows are in registers
+  // (which is why the tile before decides).  38M rows of 16 bytes, us a call, always by lane / as
+  // here, by rows per group: 1 1010 / 541, 2 490 / 371, 3 364 / 366, 4 406 / 410, 10 281 / 281,
+  // 75 183 / 179.
   const bool narrow = a.out_key_bytes == 4 && TR * 16 <= TILE_BYTES;
 
   auto issue = [&](uint64_t i) {
@@ -1035,6 +1037,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) reduce_warps_kernel(const __gri
     // still undecided (it is the last row of the previous tile)
     Key last_key = 0;
     bool pending = false;
+    bool dense = false;   // some lane held kGatherEnds heads in the tile before
     if (ntiles && t0 * TR > 0 && t0 * TR <= n) last_key = RA::global_key(a.rows, t0 * TR - 1, ks);
     for (uint64_t i = 0; i < ntiles && ok; ++i) {
       const int s = (int)(i % S);
@@ -1060,6 +1063,11 @@ __global__ void __launch_bounds__(WARPS * 32, 2) reduce_warps_kernel(const __gri
 #pragma unroll
         for (uint32_t j = 0; j < IPT; ++j) RA::read(st, lane * IPT + j, ks, vs, vmask, key[j], val[j]);
         __syncwarp();   // the rows are in registers
+        const bool gather = dense;
+        if (!gather && lane == 0 && i + S < ntiles) {
+          fence_proxy_async_smem();
+          issue(i + S);   // refill the stage
+        }
         Key pk = shfl_key(key[IPT - 1], lane ? lane - 1 : 0);
         const Key nk = shfl_key(key[0], lane < 31 ? lane + 1 : 31);
         if (lane == 0) pk = last_key;
@@ -1071,11 +1079,6 @@ __global__ void __launch_bounds__(WARPS * 32, 2) reduce_warps_kernel(const __gri
           heads |= (uint32_t)h << j;
           acc = h ? val[j] : acc + val[j];
           racc[j] = acc;
-        }
-        const bool gather = narrow && __reduce_max_sync(0xffffffffu, (uint32_t)__popc(heads)) >= kGatherEnds;
-        if (!gather && lane == 0 && i + S < ntiles) {
-          fence_proxy_async_smem();
-          issue(i + S);   // refill the stage
         }
         if (lane == 0 && pending && (heads & 1u)) emit(direct, base, run.f, last_key, run.v, first - 1, run.h);
         uint32_t fh = heads ? ((uint32_t)__popc(heads) << 16) | (lane * IPT + 31u - __clz(heads)) : 0u;
@@ -1179,6 +1182,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) reduce_warps_kernel(const __gri
                  hb ? first + (31u - __clz(hb)) : ch);
           }
         }
+        dense = narrow && __any_sync(0xffffffffu, (uint32_t)__popc(heads) >= kGatherEnds);
         run.f += tfh >> 16;
         run.v = (tfh >> 16) ? tv : run.v + tv;
         run.h = (tfh >> 16) ? tile_row + (tfh & 0xffffu) : run.h;
