@@ -32,6 +32,7 @@
 // inside it at its final index, and leaves the partial before its first head and the partial
 // from its last head for the fix-up, which closes the runs crossing units.
 //
+#include <algorithm>
 #include <cstring>
 
 #include "host_common.h"
@@ -840,8 +841,10 @@ __global__ void sum_u32_kernel(const uint32_t* v, uint64_t n, uint32_t* out) {
 // ------------------------------------------------------------------ host side
 // Elements per unit: one unit per resident warp of the main pass where that gives full units
 // (32 warps on each of 148 SMs), fewer elements for short inputs.
+constexpr uint64_t kF64Warps = 32 * 148;
+
 uint32_t f64_unit_items(uint64_t n) {
-  const uint64_t per = (n + 32 * 148 - 1) / (32 * 148);
+  const uint64_t per = (n + kF64Warps - 1) / kF64Warps;
   const uint64_t steps = (per + kF64Step - 1) / kF64Step;
   return (uint32_t)(steps * kF64Step < kF64UnitMost ? steps * kF64Step : kF64UnitMost);
 }
@@ -862,7 +865,11 @@ struct F64Layout {
 };
 
 F64Layout f64_layout(void* ws, uint64_t n) {
-  const uint64_t unit = f64_unit_items(n), units = unit ? (n + unit - 1) / unit : 0;
+  const uint64_t unit = f64_unit_items(n);
+  // room for as many units as any smaller input makes (up to one per resident warp while units
+  // of 256 elements give no more), so that a workspace serves every smaller input too
+  const uint64_t fewest = (n + kF64Step - 1) / kF64Step;
+  const uint64_t units = std::max(unit ? (n + unit - 1) / unit : 0, std::min(fewest, kF64Warps));
   constexpr size_t partial = sizeof(SumOp<kWideLimbs>::P);   // the largest
   static_assert(partial % 16 == 0 || partial % 8 == 0, "aligned partials");
   F64Layout l;

@@ -353,3 +353,23 @@ def test_runs_over_many_units(cuda, kind, units):
             ok, ov, g = R.reduce_f64(_dev(keys, cuda), _dev(vals, cuda), R.F64_SUM)
             ek, es = O.reduce_f64_exact(keys, vals)
         assert g == es.shape[0] and np.array_equal(to_np(ok), ek) and _same_bits(to_np(ov), es), (lead, tail)
+
+
+def test_smaller_inputs_in_the_workspace_of_more(cuda):
+    """One workspace, sized for the most rows, serves the sizes around each change of unit."""
+    import torch
+    most = 2_000_000
+    wsb = R.LIB.rfx_reduce_f64_workspace(most)
+    ws = R._empty_bytes(wsb, cuda)
+    keys, vals = gen_keys(4, most, 500, 1), gen_values("prices", most, 2)
+    vals[5] = 1e-40   # the widest partials too
+    dk, dv = _dev(keys, cuda), _dev(vals, cuda)
+    ok, ov = torch.empty_like(dk), torch.empty_like(dv)
+    g = torch.zeros(1, dtype=torch.int64, device=cuda)
+    for n in (most, 4736 * 256 + 1, 4736 * 256, 4736 * 256 - 1, 300, 1):
+        st = R.LIB.rfx_reduce_f64(R._ptr(dk), n, 4, R._ptr(dv), R.F64_SUM, R._ptr(ok), R._ptr(ov), R._ptr(g), R._ptr(ws),
+                                  wsb, R._stream())
+        assert st == R.OK, n
+        k = int(g.item())
+        ek, es = O.reduce_f64_exact(keys[:n], vals[:n])
+        assert k == es.shape[0] and np.array_equal(to_np(ok[:k]), ek) and _same_bits(to_np(ov[:k]), es), n
