@@ -12,14 +12,14 @@ rfx_status run_sort(SortPlan&, uint32_t);
 template <int K>
 rfx_status run_cluster(const ClusterSort&, uint32_t);
 template <int K>
-uint64_t sort_tiles_for(uint64_t, uint32_t);
+SortTiles sort_tiles_for(uint64_t, uint32_t);
 
 namespace {
 
 bool valid_width(uint32_t k) { return k == 1 || k == 2 || k == 4 || k == 8 || k == 16 || k == 32 || k == 64; }
 bool valid_vwidth(uint32_t v) { return v == 0 || v == 1 || v == 2 || v == 4 || v == 8 || v == 16; }
 
-uint64_t tiles_for(uint32_t kb, uint64_t n, uint32_t vb) {
+SortTiles tiles_for(uint32_t kb, uint64_t n, uint32_t vb) {
   switch (kb) {
     case 1: return sort_tiles_for<1>(n, vb);
     case 2: return sort_tiles_for<2>(n, vb);
@@ -74,7 +74,8 @@ SortLayout layout(void* ws, uint64_t n, uint32_t kb, uint32_t vb, uint32_t begin
   SortLayout L;
   const uint32_t bits = end_bit - begin_bit;
   L.passes = std::min<uint32_t>((std::min<uint32_t>(bits, 128) + 7) / 8, kMaxSortPasses);
-  L.tiles = tiles_for(kb, n, vb);
+  const SortTiles tiles = tiles_for(kb, n, vb);
+  L.tiles = tiles.tiles;
   Carver c(ws);
   L.alt_keys = c.take<uint8_t>(n * kb);
   L.alt_vals = c.take<uint8_t>(vb ? n * vb : 0);
@@ -85,7 +86,7 @@ SortLayout layout(void* ws, uint64_t n, uint32_t kb, uint32_t vb, uint32_t begin
   const size_t ctrl_start = c.used;
   L.ctrl = c.take<uint32_t>(kMaxSortPasses * kRadix + 2 * kMaxSortPasses + 1);
   L.ctrl_bytes = c.used - ctrl_start;
-  L.status = c.take<uint32_t>((size_t)L.passes * L.tiles * kRadix);
+  L.status = c.take<uint32_t>((size_t)L.passes * tiles.most * kRadix);
   L.total = align_up(c.used, 256);
   return L;
 }

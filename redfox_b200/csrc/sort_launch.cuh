@@ -2,6 +2,8 @@
 // sort_k{1,2,4,8,16,32,64}.cu.
 #pragma once
 
+#include <algorithm>
+
 #include "host_common.h"
 #include "sort_cluster.cuh"
 #include "sort_kernels.cuh"
@@ -31,6 +33,11 @@ struct SortPlan {
   cudaStream_t stream;
 };
 
+struct SortTiles {
+  uint64_t tiles;
+  uint64_t most;
+};
+
 struct ClusterSort {
   const uint8_t* keys_in;
   const uint8_t* vals_in;
@@ -51,6 +58,15 @@ template <int K, int V>
 uint64_t sort_tiles(uint64_t n) {
   const uint64_t tile = sort_small<K, V>(n) ? SortTuning<K, V, kSortHasSmall<K, V>>::TILE : SortTuning<K, V>::TILE;
   return (n + tile - 1) / tile;
+}
+
+// The most tiles that any input of up to n elements makes: a workspace with look-back words
+// for that many serves them all.
+template <int K, int V>
+uint64_t sort_tiles_most(uint64_t n) {
+  constexpr uint64_t kSmallMost = kSortHasSmall<K, V> ? kSortSmallBelow * SortTuning<K, V>::TILE : 0;
+  const uint64_t tiles = sort_tiles<K, V>(n);
+  return n > kSmallMost ? std::max(tiles, sort_tiles<K, V>(kSmallMost)) : tiles;
 }
 
 // Histogram of every digit; clears the look-back words.
@@ -178,21 +194,22 @@ rfx_status run_sort(SortPlan& s, uint32_t vbytes) {
   }
 }
 
+// The tiles of n elements, and the most of up to n.
 template <int K>
-uint64_t sort_tiles_for(uint64_t n, uint32_t vbytes) {
+SortTiles sort_tiles_for(uint64_t n, uint32_t vbytes) {
   switch (vbytes) {
-    case 0: return sort_tiles<K, 0>(n);
-    case 1: return sort_tiles<K, 1>(n);
-    case 2: return sort_tiles<K, 2>(n);
-    case 4: return sort_tiles<K, 4>(n);
-    case 8: return sort_tiles<K, 8>(n);
-    default: return sort_tiles<K, 16>(n);
+    case 0: return {sort_tiles<K, 0>(n), sort_tiles_most<K, 0>(n)};
+    case 1: return {sort_tiles<K, 1>(n), sort_tiles_most<K, 1>(n)};
+    case 2: return {sort_tiles<K, 2>(n), sort_tiles_most<K, 2>(n)};
+    case 4: return {sort_tiles<K, 4>(n), sort_tiles_most<K, 4>(n)};
+    case 8: return {sort_tiles<K, 8>(n), sort_tiles_most<K, 8>(n)};
+    default: return {sort_tiles<K, 16>(n), sort_tiles_most<K, 16>(n)};
   }
 }
 
 #define RFX_INSTANTIATE_SORT(K)                                  \
   template rfx_status run_sort<K>(SortPlan&, uint32_t);          \
   template rfx_status run_cluster<K>(const ClusterSort&, uint32_t); \
-  template uint64_t sort_tiles_for<K>(uint64_t, uint32_t);
+  template SortTiles sort_tiles_for<K>(uint64_t, uint32_t);
 
 }  // namespace rfx

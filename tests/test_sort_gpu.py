@@ -311,3 +311,23 @@ def test_sort_small_and_large_tiles(cuda, kb, vb, where):
     if vb:
         assert np.array_equal(to_np(dv), exp[1])
     assert R.device_status() == R.OK
+
+
+@pytest.mark.parametrize("kb,vb", [(4, 0), (8, 0), (4, 8), (16, 0)])
+def test_smaller_inputs_in_the_workspace_of_more(cuda, kb, vb):
+    """One workspace, sized for some more rows than take small tiles, serves the sizes on either
+    side of that line."""
+    line = 148 * TILE_KEYS[kb, vb]
+    s = R.Sorter(line + 1, kb, vb, kb * 8 - 24, kb * 8)
+    for n in (line + 1, line, line - 1, line // 2, 5):
+        keys = _keys(n, kb, seed=n)
+        vals = np.random.default_rng(n).integers(0, 256, (n, vb), dtype=np.uint8) if vb else None
+        s.n = n
+        dk, dv = _dev(keys, cuda), _dev(vals, cuda) if vb else None
+        s(dk, dv)
+        exp = (O.sort_pairs(keys, vals, begin_bit=s.begin, end_bit=s.end, threads=8) if vb
+               else (O.sort_pairs(keys, begin_bit=s.begin, end_bit=s.end, threads=8), None))
+        assert np.array_equal(to_np(dk), exp[0]), n
+        if vb:
+            assert np.array_equal(to_np(dv), exp[1]), n
+    assert R.device_status() == R.OK
