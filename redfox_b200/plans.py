@@ -118,17 +118,18 @@ def three_relation(d1, d2, f, list_in, list_out, f_sorted=None, stream=None):
     sorted as part of the plan."""
     import torch
     d1s, _ = R.select(d1, [32, 8], [(R.EQ, (R.OPND_VAR, 1), (R.OPND_CONST, C2_SEGMENT), R.I8)], stream=stream)
-    d2s, _ = R.select_project(d2, [32, 32, 32], [(R.GE, (R.OPND_VAR, 2), (R.OPND_CONST, C2_DATE_LO), R.I32),
+    # what a sort reads keeps a name until the end: the sorts run in the order of `stream`
+    d2u, _ = R.select_project(d2, [32, 32, 32], [(R.GE, (R.OPND_VAR, 2), (R.OPND_CONST, C2_DATE_LO), R.I32),
                                                  (R.LT, (R.OPND_VAR, 2), (R.OPND_CONST, C2_DATE_HI), R.I32)],
                               [], [32, 32], [1, 0], stream=stream)                     # (fk, pk)
-    d2s, _ = R.sorted_copy(d2s, begin_bit=32, end_bit=64, stream=stream)               # on fk
+    d2s, _ = R.sorted_copy(d2u, begin_bit=32, end_bit=64, stream=stream)               # on fk
     j1, _ = R.join_tuples_two_step(d1s, 8, d2s, 32, 16, stream=stream)                 # (pk1, seg, pk2)
-    keys = R.project(j1, [32, 8, 32], [32], [2], stream=stream).view(torch.int32).view(-1)
-    keys, _ = R.sorted_copy(keys, stream=stream)
+    unsorted = R.project(j1, [32, 8, 32], [32], [2], stream=stream).view(torch.int32).view(-1)
+    keys, _ = R.sorted_copy(unsorted, stream=stream)
     keys = R.set_op(R.SET_INTERSECTION, keys, list_in, stream=stream)
     keys = R.set_op(R.SET_DIFFERENCE, keys, list_out, stream=stream)
     if f_sorted is None:
-        f = _packed(f)   # held until the end: the sort reads it in stream order
+        f = _packed(f)
         f_sorted, _ = R.sorted_copy(f, begin_bit=64, end_bit=96, stream=stream)       # on fk
     keys4 = keys.view(torch.uint8).view(-1, 4)
     j2, total = R.join_tuples_two_step(keys4, 0, f_sorted, 64, 16, stream=stream)     # (pk2, amount)
