@@ -272,3 +272,34 @@ extern "C" rfx_status rfx_mgpu_sort_key(void* keys, uint64_t n, uint64_t key_typ
   if (!kb) return RFX_ERR_UNSUPPORTED;
   return sort_sync(keys, nullptr, n, kb, 0, 0, kb * 8);
 }
+
+// ------------------------------------------------------------------ for the tests
+// Parts of the sort that no input reaches on demand; not declared in rfx.h.
+namespace rfx {
+namespace {
+
+constexpr uint32_t kOrderTestMost = 12288;   // entries: 48 KB
+
+__global__ void order_entries_kernel(uint32_t* entries, uint32_t count) {
+  extern __shared__ uint32_t s_entries[];
+  for (uint32_t i = threadIdx.x; i < count; i += blockDim.x) s_entries[i] = entries[i];
+  __syncthreads();
+  order_entries(s_entries, count, blockDim.x);
+  for (uint32_t i = threadIdx.x; i < count; i += blockDim.x) entries[i] = s_entries[i];
+}
+
+}  // namespace
+}  // namespace rfx
+
+// The route of pass `pass` (sort_plan).
+extern "C" uint32_t rfx_test_sort_plan(uint32_t moving, uint32_t passes, uint32_t in_place, uint32_t pass) {
+  return sort_plan(moving, passes, in_place != 0, pass);
+}
+
+// The repair of a tile's entries, by one block (order_entries).
+extern "C" rfx_status rfx_test_order_entries(uint32_t* entries, uint32_t count, uint32_t threads, void* stream) {
+  if (!entries || count > kOrderTestMost || threads == 0 || threads > 1024 || threads % 32) return RFX_ERR_INVALID;
+  order_entries_kernel<<<1, threads, count * sizeof(uint32_t), as_stream(stream)>>>(entries, count);
+  RFX_CUDA_TRY(cudaGetLastError());
+  return RFX_OK;
+}

@@ -134,8 +134,16 @@ __device__ __forceinline__ uint32_t elem_bits(const Elem<K>& e, uint32_t shift) 
 constexpr uint32_t kRouteSort = 16;
 constexpr uint32_t kRouteCopy = 32;
 
-__device__ constexpr uint32_t sort_route(uint32_t what, uint32_t from, uint32_t to) {
+__host__ __device__ constexpr uint32_t sort_route(uint32_t what, uint32_t from, uint32_t to) {
   return what | from | to << 2;
+}
+
+__host__ __device__ __forceinline__ uint32_t bit_count(uint32_t x) {
+#ifdef __CUDA_ARCH__
+  return __popc(x);
+#else
+  return (uint32_t)__builtin_popcount(x);
+#endif
 }
 
 // The part of pass p of `passes`; bit p of `moving`: pass p's digits are not all the same.
@@ -143,21 +151,22 @@ __device__ constexpr uint32_t sort_route(uint32_t what, uint32_t from, uint32_t 
 // copies it back; it always runs).  An even number of passes that move keys goes back and
 // forth between 1 and 2; in place an odd number from 3 on takes 2, 3, 1 first; a single one
 // is copied, before or after, by a pass that moves nothing itself.
-__device__ __forceinline__ uint32_t sort_plan(uint32_t moving, uint32_t passes, bool in_place, uint32_t p) {
+__host__ __device__ __forceinline__ uint32_t sort_plan(uint32_t moving, uint32_t passes, bool in_place, uint32_t p) {
   if (passes == 1) moving = 1;
-  const uint32_t m = __popc(moving), last = 31 - __clz(moving);
+  const uint32_t m = bit_count(moving);
   if (m == 0) return !in_place && p == passes - 1 ? sort_route(kRouteCopy, 0, 1) : 0u;
+  const bool moves = moving >> p & 1;
   if (in_place && m == 1 && passes > 1) {
-    if (last < passes - 1)
-      return p == last ? sort_route(kRouteSort, 0, 2) : p == passes - 1 ? sort_route(kRouteCopy, 2, 1) : 0u;
-    return p == last ? sort_route(kRouteSort, 2, 1) : p == 0 ? sort_route(kRouteCopy, 0, 2) : 0u;
+    if (!(moving >> (passes - 1) & 1))
+      return moves ? sort_route(kRouteSort, 0, 2) : p == passes - 1 ? sort_route(kRouteCopy, 2, 1) : 0u;
+    return moves ? sort_route(kRouteSort, 2, 1) : p == 0 ? sort_route(kRouteCopy, 0, 2) : 0u;
   }
-  if (!(moving >> p & 1)) return 0;
+  if (!moves) return 0;
   auto to = [&](uint32_t j) -> uint32_t {   // of the j-th pass that moves
     if (!in_place || m % 2 == 0) return (m - 1 - j) % 2 ? 2 : 1;
     return j == 1 ? 3 : j == 0 || j % 2 ? 2 : 1;
   };
-  const uint32_t j = __popc(moving & ((1u << p) - 1));
+  const uint32_t j = bit_count(moving & ((1u << p) - 1));
   return sort_route(kRouteSort, j ? to(j - 1) : 0u, to(j));
 }
 

@@ -331,3 +331,58 @@ def test_smaller_inputs_in_the_workspace_of_more(cuda, kb, vb):
         if vb:
             assert np.array_equal(to_np(dv), exp[1]), n
     assert R.device_status() == R.OK
+
+
+@pytest.mark.parametrize("threads", [256, 512])
+@pytest.mark.parametrize("count", [0, 1, 2, 3, 31, 255, 257, 511, 513, 1023, 4608, 7167, 10240])
+def test_order_entries(cuda, count, threads):
+    """The repair of a tile whose entries (digit << 16 | place in the tile) are out of order, which
+    inputs bring about only if the hardware serves a warp's atomics out of lane order: equal digits
+    exchanged within a warp's step, each digit's places turned round, one entry far off, none."""
+    import ctypes as C
+    rng = np.random.default_rng(count + threads)
+    digit = np.sort(rng.integers(0, 40, count)).astype(np.uint32)
+    want = digit << 16 | np.arange(count, dtype=np.uint32)
+    swapped, turned, far = want.copy(), want.copy(), want.copy()
+    for i in range(0, count - 31, 32):
+        part = swapped[i:i + 32]
+        for d in np.unique(part >> 16):
+            m = part >> 16 == d
+            part[m] = rng.permutation(part[m])
+    for d in np.unique(digit):
+        turned[digit == d] = turned[digit == d][::-1]
+    if count > 2:
+        far[0], far[-1] = want[-1], want[0]
+    for got in (want, swapped, turned, far):
+        dev = _dev(np.append(got, np.uint32(0xABCD)).view(np.int32), cuda)   # one more: not touched
+        st = R.LIB.rfx_test_order_entries(R._ptr(dev), C.c_uint32(count), C.c_uint32(threads), R._stream())
+        out = to_np(dev).view(np.uint32)
+        assert st == R.OK and np.array_equal(out[:count], np.sort(want)) and out[count] == 0xABCD
+
+
+@pytest.mark.parametrize("moving", [[], [0], [1], [3], [0, 3], [0, 1, 2], [1, 2, 3], [0, 1, 2, 3]])
+@pytest.mark.parametrize("kb,vb,n", [(4, 0, 70_011), (8, 4, 70_001), (4, 1, 70_003), (8, 16, 70_001)])
+def test_sort_skips_constant_digits_above_the_cluster_sort(cuda, kb, vb, n, moving):
+    """Constant digits in every place among four, sizes that the digit passes take: keys and values
+    in place and out of place, with 16-byte aligned arrays and with others."""
+    rng = np.random.default_rng(n + sum(moving))
+    keys = np.full((n + 1, kb), 0x5A, np.uint8)
+    for b in moving:
+        keys[:, kb - 4 + b] = rng.integers(0, 256, n + 1, dtype=np.uint8)
+    if kb > 4:
+        keys[:, 0] = rng.integers(0, 256, n + 1, dtype=np.uint8)   # payload: shows the order of equal keys
+    vals = rng.integers(0, 256, (n + 1, vb), dtype=np.uint8) if vb else None
+    begin, end = (kb - 4) * 8, kb * 8
+    for first in (0, 1):
+        hk, hv = keys[first:first + n], vals[first:first + n] if vb else None
+        exp = O.sort_pairs(hk, hv, begin_bit=begin, end_bit=end) if vb else (O.sort_pairs(hk, begin_bit=begin,
+                                                                                          end_bit=end), None)
+        a, av = _dev(keys, cuda)[first:first + n], _dev(vals, cuda)[first:first + n] if vb else None
+        b, bv = R.sorted_copy(a, av, begin_bit=begin, end_bit=end)
+        assert np.array_equal(to_np(a), hk)
+        R.sort_pairs(a, av, begin_bit=begin, end_bit=end)
+        for k, v in ((a, av), (b, bv)):
+            assert np.array_equal(to_np(k), exp[0]), first
+            if vb:
+                assert np.array_equal(to_np(v), exp[1]), first
+    assert R.device_status() == R.OK
