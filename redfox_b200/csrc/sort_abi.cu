@@ -134,6 +134,13 @@ rfx_status sort_pairs_impl(void* keys, void* vals, uint64_t n, uint32_t kb, uint
   small.begin_bit = begin_bit;
   small.end_bit = end_bit;
   small.stream = stream;
+  // the one-launch form needs no error word, but a program may warm up with a small sort and then
+  // capture a large one, which cannot allocate it
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess)
+    (void)cudaGetLastError();
+  else if (capture == cudaStreamCaptureStatusNone && !device_error_word())
+    return RFX_ERR_CUDA;
   const rfx_status one = dispatch_cluster(kb, small, vb);
   if (one != RFX_ERR_UNSUPPORTED) return one;
   uint32_t* err = device_error_word();

@@ -386,3 +386,33 @@ def test_sort_skips_constant_digits_above_the_cluster_sort(cuda, kb, vb, n, movi
             if vb:
                 assert np.array_equal(to_np(v), exp[1]), first
     assert R.device_status() == R.OK
+
+
+def test_a_small_sort_warms_up_for_a_captured_large_one():
+    """In a process whose first call is a small sort (the one-launch form, which needs none of the
+    device's lasting state), a larger one can be captured, as after any other first sort; a small
+    one can be captured as the first call."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import torch
+from redfox_b200 import rfx as R
+def capture(n):
+    k = torch.randint(0, 256, (n, 4), dtype=torch.uint8, device="cuda")
+    o, s, g = torch.empty_like(k), R.Sorter(n, 4), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        s(o, src_keys=k)
+    g.replay()
+    torch.cuda.synchronize()
+    return k, o
+pairs = [capture(5000)] if FIRST else []
+R.sorted_copy(torch.randint(0, 256, (5000, 4), dtype=torch.uint8, device="cuda"))
+pairs.append(capture(300000))
+assert all(torch.equal(o, R.sorted_copy(k)[0]) for k, o in pairs)
+"""
+    repo = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    for first in ("False", "True"):
+        r = subprocess.run([sys.executable, "-c", code.replace("FIRST", first)], cwd=repo, capture_output=True, text=True,
+                           timeout=300)
+        assert r.returncode == 0, (first, r.stderr[-2000:])
