@@ -151,7 +151,7 @@ rfx_status rfx_filter_aggregate(const void* in, uint64_t n, const rfx_tuple* in_
 #define RFX_SORT_SKIP_TRIVIAL 1u
 
 /* Workspace of rfx_sort_pairs: the alternate key/value buffers plus histogram and
- * look-back words. */
+ * look-back words.  Never less than for a smaller n. */
 size_t rfx_sort_workspace(uint64_t n, uint32_t key_bytes, uint32_t value_bytes,
                           uint32_t begin_bit, uint32_t end_bit);
 
@@ -298,7 +298,7 @@ rfx_status rfx_plan_schema(const rfx_plan* plan, const char* name, uint32_t* wid
 /* Operations of rfx_reduce_f64. */
 enum { RFX_F64_SUM = 0, RFX_F64_MIN = 1 };
 
-size_t rfx_reduce_f64_workspace(uint64_t n);
+size_t rfx_reduce_f64_workspace(uint64_t n);   /* never less than for a smaller n */
 
 /* Reduce-by-key over double values: thrust::reduce_by_key with plus<double>
  * (total_{8,16,32,64,128}_double, Reduce.cu:819-1453) or minimum<double> (min_32_double,
@@ -310,9 +310,11 @@ size_t rfx_reduce_f64_workspace(uint64_t n);
  * error).  NaN if a term is NaN or both infinities occur, an infinity if one occurs, -0
  * only when every term is -0.  RFX_F64_MIN is the reference's fold acc = acc < v ? acc : v
  * bit for bit (a later equal element replaces an earlier one; a NaN replaces the
- * accumulator and the next element replaces the NaN).  Stream-ordered; a value whose bits
- * fall more than 2^107 below the largest one makes a second, full-range pass do the work
- * (decided on the device).  n < 2^30. */
+ * accumulator and the next element replaces the NaN).  Stream-ordered.  A sum is kept in a
+ * pair of doubles; where that loses bits (a run's values spanning more than about 100 binary
+ * places, or a finite value from 2^1000 on) a second pass works in 192-bit integers, and where
+ * a value's bits fall more than 2^107 below the largest one a third, full-range pass does the
+ * work (both decided on the device).  n < 2^30. */
 rfx_status rfx_reduce_f64(const void* keys, uint64_t n, uint32_t key_bytes, const double* values,
                           uint32_t op, void* out_keys, double* out_values, uint64_t* d_groups,
                           void* workspace, size_t workspace_bytes, void* stream);

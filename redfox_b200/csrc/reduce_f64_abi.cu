@@ -568,10 +568,11 @@ __global__ void __launch_bounds__(256) f64_emax(F64Args a) {
 // (16-byte loads).  A lane folds its elements, writing the runs that start and end among
 // them; a segmented warp scan gives every lane what is open before it.  Bound by the latency
 // of a step's chain (loads, fold, scan), so by the warps resident: 19.3M elements, 256K runs,
-// SUM with 32 warps per SM (64 registers, 16 bytes of spills) 85 us, with 24 warps 105, with 16
-// warps and the next step's loads in flight 106, the 3-limb integers 152; MIN 73 / 98 / 90,
-// before 100.  A column that the pair cannot hold is found out in the first steps and costs the
-// pair's pass 15 us (values over 80 binary places), one such value in the middle 30.
+// SUM with 32 warps per SM (64 registers, 16 bytes of spills) 91 us, MIN 67, the 3-limb integers
+// with 16 warps 152.  An earlier form of the pair took 87 with 32 warps, 105 with 24, 106 with 16
+// and the next step's loads in flight.  A column that the pair cannot hold is found out in the
+// first steps and costs the pair's pass 15 us (values over 80 binary places), one such value in
+// the middle 30.
 template <int KB, class Op>
 __global__ void __launch_bounds__(256, Op::BLOCKS) f64_unit_kernel(F64Args a, uint64_t units) {
   grid_wait();   // chained launch

@@ -22,7 +22,8 @@ constexpr int kSortLookWindow = 8;  // predecessors examined per look-back round
 // a tile as their shared memory allows (the per-tile costs -- barriers, the look-back -- and
 // the number of digit runs a tile is written in fall with its size), over as many threads as
 // that leaves registers for.  Whole sorts of four passes, us, at 1M / 4M / 60M elements:
-//   4 B   512 x 20: 63 / 117 / 942; 512 x 22: 68 / 122 / 930; 384 x 28: 74 / 133 / 1060
+//   4 B   512 x 20: 63 / 117 / 942 (64 registers, 28 bytes of spills); 512 x 22: 68 / 122 / 930;
+//         384 x 28: 74 / 133 / 1060
 //   8 B   512 x 14: 62 / 120 / 1170; 512 x 12: 62 / 125 / 1211; 384 x 16: 62 / 138 / 1281
 //   4 B keys with 8 B values   512 x 10: 65 / 141 / 1447; 384 x 12: 63 / 148 / 1510; 384 x 16: 71 / 153 / 1389
 //   16 B  512 x 9: 67 / 162 / 1688; 512 x 8: 65 / 166 / 1746; 384 x 12: 71 / 167 / 1710
@@ -104,25 +105,6 @@ __device__ __forceinline__ void store_elem(uint8_t* base, uint64_t i, const Elem
     uint4* p = reinterpret_cast<uint4*>(base + i * B);
 #pragma unroll
     for (int k = 0; k < B / 16; ++k) p[k] = make_uint4(e.w[4 * k], e.w[4 * k + 1], e.w[4 * k + 2], e.w[4 * k + 3]);
-  }
-}
-
-// Bits [shift, shift + 8) of the element (the caller masks to the digit width).
-template <int K>
-__device__ __forceinline__ uint32_t elem_bits(const Elem<K>& e, uint32_t shift) {
-  if constexpr (Elem<K>::NW == 1) {
-    return e.w[0] >> shift;
-  } else {
-    const uint32_t q = shift >> 5;
-    uint32_t lo = e.w[0], hi = e.w[1];
-#pragma unroll
-    for (int k = 1; k < Elem<K>::NW; ++k) {
-      if ((int)q == k) {
-        lo = e.w[k];
-        hi = k + 1 < Elem<K>::NW ? e.w[k + 1] : 0u;
-      }
-    }
-    return __funnelshift_r(lo, hi, shift & 31);
   }
 }
 

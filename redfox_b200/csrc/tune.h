@@ -24,7 +24,7 @@ enum TuneOp : uint32_t {
                           // with 8, 4 or 16
   TUNE_SCAN_COMPACT = 3,  // plan-specialised select / project: items per thread
   TUNE_SCAN_AGGREGATE = 4,  // plan-specialised filter-aggregate: rows per thread per iteration
-  TUNE_SORT_PASS = 5,     // the sort's digit pass: a single form, nothing asks for it
+                          // (5 was the sort's digit pass, which has a single form now)
   TUNE_JOIN_EMIT = 6,     // fused join emit: operands staged in shared memory by bulk copies, or gathered
 };
 

@@ -626,7 +626,7 @@ _declare_tune()
 TUNE_OPS = {1: "reduce_tuples", 2: "set_filter", 3: "select_compact", 4: "filter_aggregate", 5: "sort_pass",
             6: "join_emit"}
 TUNE_JOIN_EMIT = 6   # variants: 0 operands staged in shared memory by bulk copies, 1 gathered per output
-TUNE_SORT_PASS = 5   # the sort has one digit pass: pinning it changes nothing
+TUNE_SORT_PASS = 5   # kept for its callers: the sort has one digit pass, nothing reads this id
 
 
 def tune(mode=1):
