@@ -9,13 +9,14 @@
 //     the flag stays down hi + lo is the exact sum whatever the order of the additions, and
 //     one rounding of hi + lo finishes it.  This holds for values whose bits span about 100
 //     binary places, such as amounts of money, with or without infinities and NaNs.
-//   * If the flag went up (a wider span, a finite value from 2^1000 on), a second pass
-//     works in integers: every double is a 53-bit integer times a power of two, so a run's
-//     sum is accumulated as a two's-complement integer in units of 2^L over W 64-bit limbs
-//     (add with carry).  W = 3 limbs with L set from the largest exponent in the input: exact
-//     for every value within 2^107 of the largest, with room for 2^30 terms.
+//   * Where the flag went up (a wider span, a finite value from 2^1000 on), a second pass sums
+//     the runs that lost bits again, in integers: every double is a 53-bit integer times a
+//     power of two, so a run's sum is accumulated as a two's-complement integer in units of 2^L
+//     over W 64-bit limbs (add with carry).  W = 3 limbs with L set from the largest exponent in
+//     the units that are summed again: exact for every value within 2^107 of the largest, with
+//     room for 2^30 terms.
 //   * A value below that window with bits that would be lost raises a flag too, and a third
-//     pass with W = 34 limbs and L = -1074, which covers every finite double, runs.
+//     pass with W = 34 limbs and L = -1074, which covers every finite double, does the same.
 // The kernels of the later passes are always enqueued and return at once unless their flag is
 // set, so no host round trip is needed.  Specials follow IEEE addition: NaN if any NaN or both
 // infinities, else the infinity, and an exact zero is -0 only when every term is -0.
@@ -31,7 +32,6 @@
 // pass folds a unit in registers and warp shuffles, writes every run that starts and ends
 // inside it at its final index, and leaves the partial before its first head and the partial
 // from its last head for the fix-up, which closes the runs crossing units.
-//
 #include <algorithm>
 #include <cstring>
 
@@ -51,9 +51,10 @@ enum : uint32_t { kSumNaN = 1, kSumPosInf = 2, kSumNegInf = 4, kSumNotNegZero = 
 // W 64-bit limbs holding a two's-complement integer (limb 0 lowest) in units of 2^L.
 // Additions are exact modulo 2^(64W); the true sum stays inside the signed range by the
 // choice of L, so the result is exact and independent of the order of the additions.
+// TENTATIVE: the pass finds out where it loses bits; AGAIN: the pass does those units over.
 template <int W>
 struct SumOp {
-  static constexpr bool TENTATIVE = false;
+  static constexpr bool TENTATIVE = false, AGAIN = true;
   static constexpr bool COMMUTES = W == 3;   // (the 34 limbs are not worth another copy)
   static constexpr int BLOCKS = W == 3 ? 2 : 1;   // of 256 threads per SM: the limbs live in registers
   struct P {
@@ -221,7 +222,7 @@ struct SumOp {
 // them.  The errors are NaN from there on and say nothing.
 struct PairOp {
   static constexpr int BLOCKS = 4;
-  static constexpr bool TENTATIVE = true;   // the pass gives up once a flag is up
+  static constexpr bool TENTATIVE = true, AGAIN = false;
   static constexpr bool COMMUTES = true;
   struct P {
     double hi, lo;
@@ -264,7 +265,7 @@ struct PairOp {
 // ------------------------------------------------------------------ minimum (the fold)
 struct MinOp {
   static constexpr int BLOCKS = 4;
-  static constexpr bool TENTATIVE = false;
+  static constexpr bool TENTATIVE = false, AGAIN = false;
   static constexpr bool COMMUTES = false;
   struct P {
     unsigned long long v;  // bits of the fold value (a NaN while pending)
@@ -381,12 +382,17 @@ struct F64Args {
   uint32_t* base;       // index of the unit's first run (heads before it)
   void* first;          // Op::P per unit: before its first head (the whole unit if it has none)
   void* last;           // Op::P per unit: from its last head
+  uint32_t* need;       // per unit: what the integer passes do over (kLossy, kInvolved, kReclose)
   int* emax;            // max biased exponent of the finite values (the 3-limb pass's window)
   int fixed_L;          // used when emax is null
-  uint32_t* inexact;    // raised when the pass could not be exact
+  uint32_t* inexact;    // raised when the pass was not exact everywhere
   const uint32_t* gate; // if set, the kernels do nothing unless *gate != 0
   uint32_t* err;
 };
+
+// Why a unit is summed again in integers: bits were lost in it; a run that lost bits goes through
+// it; that run ends at its first head (or with it).
+enum : uint32_t { kLossy = 1, kInvolved = 2, kReclose = 4 };
 
 __device__ __forceinline__ bool gated_off(const F64Args& a) { return a.gate && *a.gate == 0u; }
 
@@ -490,7 +496,10 @@ __global__ void __launch_bounds__(256) f64_unit_count(F64Args a, uint64_t units)
       c += (uint32_t)__popc(head_bits<KB>(a, k, first, e1));
     }
     c = __reduce_add_sync(0xffffffffu, c);
-    if (lane == 0) a.heads[u] = c;
+    if (lane == 0) {
+      a.heads[u] = c;
+      a.need[u] = 0;
+    }
   }
   __threadfence();
   __syncthreads();
@@ -533,46 +542,53 @@ __global__ void __launch_bounds__(256) f64_unit_count(F64Args a, uint64_t units)
   if (t == 0) *a.d_groups = carry;
 }
 
-// The largest biased exponent of the finite values (the 3-limb pass's window).
-__global__ void __launch_bounds__(256) f64_emax(F64Args a) {
+// The largest biased exponent of the finite values of the units that are summed again (the 3-limb
+// pass's window), one warp per unit, 16 bytes per load and four loads in flight.
+__global__ void __launch_bounds__(256) f64_emax(F64Args a, uint64_t units) {
   grid_wait();   // chained launch
   grid_release();
   if (gated_off(a)) return;
+  const uint32_t lane = threadIdx.x & 31;
+  const bool vec = (reinterpret_cast<uintptr_t>(a.vals) & 15u) == 0;
   int m = 1;
   auto take = [&](double x) {
     const int eb = (__double2hiint(x) >> 20) & 0x7ff;
     if (eb != 0x7ff && eb > m) m = eb;
   };
-  // 16 bytes per load, four loads in flight
-  const uint32_t tid = blockIdx.x * 256 + threadIdx.x, stride = gridDim.x * 256, n = (uint32_t)a.n;
-  const uint32_t pairs = (reinterpret_cast<uintptr_t>(a.vals) & 15u) == 0 ? n / 2 : 0u;
-  for (uint32_t c = tid; c < pairs; c += 4 * stride) {
-    double2 v[4];
+  for (uint32_t u = blockIdx.x * 8 + (threadIdx.x >> 5); u < units; u += gridDim.x * 8) {
+    if (!a.need[u]) continue;
+    const uint32_t e0 = u * a.unit, e1 = min(e0 + a.unit, (uint32_t)a.n);
+    uint32_t i = e0;
+    if (vec) {
+      for (; i + kF64Step <= e1; i += kF64Step) {
+        double2 v[4];
 #pragma unroll
-    for (uint32_t k = 0; k < 4; ++k) {
-      const uint32_t i = c + k * stride;
-      v[k] = i < pairs ? reinterpret_cast<const double2*>(a.vals)[i] : make_double2(0.0, 0.0);
-    }
+        for (int k = 0; k < 4; ++k) v[k] = reinterpret_cast<const double2*>(a.vals + i)[32 * k + lane];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      take(v[k].x);
-      take(v[k].y);
+        for (int k = 0; k < 4; ++k) {
+          take(v[k].x);
+          take(v[k].y);
+        }
+      }
     }
+    for (i += lane; i < e1; i += 32) take(a.vals[i]);
   }
-  for (uint32_t i = 2 * pairs + tid; i < n; i += stride) take(a.vals[i]);
   m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0) atomicMax(a.emax, m);
+  if (lane == 0) atomicMax(a.emax, m);
 }
 
 // The main pass: a warp folds its unit 256 elements at a time, 8 consecutive ones per lane
 // (16-byte loads).  A lane folds its elements, writing the runs that start and end among
 // them; a segmented warp scan gives every lane what is open before it.  Bound by the latency
 // of a step's chain (loads, fold, scan), so by the warps resident: 19.3M elements, 256K runs,
-// SUM with 32 warps per SM (64 registers, 16 bytes of spills) 91 us, MIN 67, the 3-limb integers
+// SUM with 32 warps per SM (64 registers, 20 bytes of spills) 91 us, MIN 67, the 3-limb integers
 // with 16 warps 152.  An earlier form of the pair took 87 with 32 warps, 105 with 24, 106 with 16
-// and the next step's loads in flight.  A column that the pair cannot hold is found out in the
-// first steps and costs the pair's pass 15 us (values over 80 binary places), one such value in
-// the middle 30.
+// and the next step's loads in flight.
+//
+// A unit in which an addition of the pair lost bits is left at the next step and marked; the
+// integer passes do the marked units over.  us a call with the integer pass alone / now: all units
+// done over (values over 80 binary places) 319 / 262, a few (one value that does not fit) 322 / 247,
+// of 60M elements and 1M runs 690 / 462, one run over 19.3M with one such value 278 / 248 to 284.
 template <int KB, class Op>
 __global__ void __launch_bounds__(256, Op::BLOCKS) f64_unit_kernel(F64Args a, uint64_t units) {
   grid_wait();   // chained launch
@@ -586,8 +602,12 @@ __global__ void __launch_bounds__(256, Op::BLOCKS) f64_unit_kernel(F64Args a, ui
   const int L = window_L(a);
   const bool vk = (reinterpret_cast<uintptr_t>(a.keys) & 15u) == 0;
   const bool vv = (reinterpret_cast<uintptr_t>(a.vals) & 15u) == 0;
-  bool bad = false;
+  // one run over everything: bits lost in any unit have all done over, so each warp looks whether
+  // another has lost some (the flag is asked for a step before it is used)
+  const bool one_run = Op::TENTATIVE && (KB == 0 || *a.d_groups == 1);
+  bool bad = false, raised = false;
   for (uint32_t u = gw; u < units; u += nw) {
+    if (Op::AGAIN && !a.need[u]) continue;
     const uint32_t e0 = u * a.unit, e1 = min(e0 + a.unit, (uint32_t)a.n);   // below 2^30
     uint32_t run_base = a.base[u];   // index of the next head's run
     P carry = Op::identity();
@@ -607,16 +627,11 @@ __global__ void __launch_bounds__(256, Op::BLOCKS) f64_unit_kernel(F64Args a, ui
         holding = false;
       }
     };
-    uint32_t raised = 0;
     for (uint32_t tb = e0; tb < e1; tb += kF64Step) {
       if constexpr (Op::TENTATIVE) {
-        // this pass is for nothing once a flag is up: this warp's, or another's, looked at
-        // every fourth step
-        if (__any_sync(0xffffffffu, bad || raised)) {
-          if (lane == 0) atomicOr(a.inexact, 1u);
-          return;
-        }
-        if ((tb / kF64Step & 3) == 3) raised = ld_relaxed_u32(a.inexact);
+        if (one_run && (tb / kF64Step & 3) == 3) bad = bad || raised;
+        if (__any_sync(0xffffffffu, bad)) break;   // the unit is done over
+        if (one_run && (tb / kF64Step & 3) == 2) raised = ld_relaxed_u32(a.inexact) != 0;
       }
       const uint32_t first = tb + lane * V;
       Key keys[V];
@@ -706,9 +721,16 @@ __global__ void __launch_bounds__(256, Op::BLOCKS) f64_unit_kernel(F64Args a, ui
       run_base += __shfl_sync(0xffffffffu, inc, 31);
     }
     release();
+    if (Op::TENTATIVE && __any_sync(0xffffffffu, bad)) {
+      if (lane == 0) {
+        a.need[u] = kLossy;
+        if (!raised) *static_cast<volatile uint32_t*>(a.inexact) = 1u;   // the only value ever written
+      }
+      bad = false;
+      continue;
+    }
     if (lane == 0) reinterpret_cast<P*>(carry_head ? a.last : a.first)[u] = carry;
   }
-  if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.inexact, 1u);
 }
 
 // The runs that cross units, one warp per unit: a unit with a head closes the run of the last
@@ -718,32 +740,33 @@ __global__ void __launch_bounds__(256, Op::BLOCKS) f64_unit_kernel(F64Args a, ui
 // by one block only.  The longest walk is one run over everything, us a call with the one warp
 // walking on by 512 / with its block: SUM of 19.3M values (4712 units) 191 / 146, of 60M 467 / 331,
 // of 200M 1398 / 855; MIN 201 / 153, 473 / 322, 1470 / 894.
+//
+// A run that loses bits here, or that goes through a unit which did, is not written: its units
+// are marked for the integer passes, which close the marked runs alone.
 template <class Op>
 __global__ void __launch_bounds__(256) f64_fix(F64Args a, uint64_t units) {
   grid_wait();   // chained launch
   grid_release();
   if (gated_off(a)) return;
-  if (Op::TENTATIVE && __syncthreads_or(ld_relaxed_u32(a.inexact) != 0)) return;
   using P = typename Op::P;
   __shared__ P s_part[8];
-  __shared__ bool s_head[8];
-  __shared__ int32_t s_pos;
+  __shared__ bool s_head[8], s_lost[8], s_again;
+  __shared__ int32_t s_stop[8], s_pos;
   const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const uint32_t u = blockIdx.x * 8 + warp;   // below 2^22
   const int L = window_L(a);
+  const uint32_t mine = u < units ? a.need[u] : 0u;
   const bool head = u < units && a.heads[u] > 0, last = u + 1 == units;
-  const bool closes = u > 0 && (head || last);   // the run that is open before the unit
+  const bool closes = u > 0 && (head || last) && (!Op::AGAIN || (mine & kReclose));   // the run open before the unit
   const P* first_of = reinterpret_cast<const P*>(a.first);
   const P* last_of = reinterpret_cast<const P*>(a.last);
-  // an addition that lost bits counts in whichever lane it was made, but only where the sum
-  // goes into the run: lanes beyond the nearest head hold units of earlier runs
-  bool bad = false, open = false;
-  P acc = Op::identity();
-  // the sum of the lanes' parts up to the nearest lane with a head, in order (a higher lane
-  // holds earlier units), in lane 0; whether there is such a lane
-  auto join = [&](P& x, bool h, bool lost, bool& lost_any) {
+  auto lossy = [&](int32_t v) { return Op::TENTATIVE && (a.need[v] & kLossy); };
+  // The sum of the lanes' parts up to the nearest lane with a head, in order (a higher lane holds
+  // earlier units), in lane 0.  `lost`: bits were lost in the lane's part; then in the sum (lanes
+  // beyond the nearest head hold units of earlier runs).  Returns that lane, 32 if there is none.
+  auto join = [&](P& x, bool h, bool& lost) -> uint32_t {
     const uint32_t m = __ballot_sync(0xffffffffu, h);
-    const uint32_t stop = m ? __ffs(m) - 1 : 31u;
+    const uint32_t stop = m ? __ffs(m) - 1 : 32u;
     if (lane > stop) {
       x = Op::identity();
       lost = false;
@@ -753,16 +776,22 @@ __global__ void __launch_bounds__(256) f64_fix(F64Args a, uint64_t units) {
       const P y = shfl_down_any(x, o);
       if ((lane & (2 * o - 1)) == 0) x = Op::combine(y, x, lost);   // the lanes that lead to lane 0
     }
-    lost_any = lost;
-    return m != 0;
+    lost = __any_sync(0xffffffffu, lost);
+    return stop;
   };
+  bool bad = false, open = false;
+  uint32_t stop = 0;
+  P acc = Op::identity();
   if (closes) {
     const int32_t v = (int32_t)u - 1 - (int32_t)lane;
     const bool h = v >= 0 && a.heads[v] > 0;
+    bad = v >= 0 && lossy(v);
     if (v >= 0) acc = h ? last_of[v] : first_of[v];
-    open = !join(acc, h, false, bad) && u > 32;
+    stop = join(acc, h, bad);
+    open = stop == 32;   // (unit 0 has a head)
   }
-  if (__syncthreads_or(open)) {
+  const bool walk = __syncthreads_or(open);
+  if (walk) {
     constexpr int R = 16;
     if (open && lane == 0) s_pos = (int32_t)u - 33;
     __syncthreads();
@@ -771,51 +800,78 @@ __global__ void __launch_bounds__(256) f64_fix(F64Args a, uint64_t units) {
       // this thread's units, the newest first, up to one with a head
       P x = Op::identity();
       bool h = false, lost = false;
-      const int32_t p0 = pos - (int32_t)t * r;
+      int32_t at = pos - (int32_t)t * r;
       if (r == 1) {
-        h = p0 >= 0 && a.heads[p0] > 0;
-        if (p0 >= 0) x = h ? last_of[p0] : first_of[p0];
+        if (at >= 0) {
+          h = a.heads[at] > 0;
+          lost = lossy(at);
+          x = h ? last_of[at] : first_of[at];
+        }
       } else {
+        const int32_t p0 = at;
 #pragma unroll(sizeof(P) <= 32 ? 8 : 1)
         for (int k = 0; k < R; ++k) {
           const int32_t v = p0 - k;
           const int32_t c = v >= 0 ? v : 0;   // loaded whether it counts or not: the loads overlap
-          const bool hk = a.heads[c] > 0;
+          const bool hk = a.heads[c] > 0, lk = lossy(c);
           const P y = hk ? last_of[c] : first_of[c];
           if (v >= 0 && !h) {
             x = Op::combine(y, x, lost);
+            lost = lost || lk;
             h = hk;
+            at = v;
           }
         }
       }
-      const bool any = join(x, h, lost, lost);
+      const uint32_t near = join(x, h, lost);
       if (lane == 0) {
         s_part[warp] = x;
-        s_head[warp] = any;
+        s_lost[warp] = lost;
+        s_head[warp] = near < 32;
       }
+      if (lane == near) s_stop[warp] = at;
       __syncthreads();
       bool found = false;
       uint32_t used = 0;   // warps up to the nearest one with a head
       for (; used < 8 && !found; ++used) {
         if (open && lane == 0) acc = Op::combine(s_part[used], acc, bad);
+        bad = bad || (open && s_lost[used]);
         found = s_head[used];
       }
-      bad = bad || (lost && warp < used);
-      pos -= 256 * r;
+      if (found) pos = s_stop[used - 1];
+      else pos -= 256 * r;
       if (found || pos < 0) break;
       __syncthreads();   // the parts are written again
     }
+    if (open && lane == 0) s_pos = pos;   // the run's first unit
   }
   if (lane == 0 && u < units) {
     const uint32_t base = a.base[u];
     if (closes) {
       const P y = Op::combine(acc, first_of[u], bad);
-      a.out_vals[base - 1] = __longlong_as_double((long long)Op::finalize(y, L));
+      bad = bad || lossy((int32_t)u);
+      if (!Op::TENTATIVE || !bad) a.out_vals[base - 1] = __longlong_as_double((long long)Op::finalize(y, L));
     }
-    if (last && head)
+    if (last && head && (Op::AGAIN ? mine != 0 : !(Op::TENTATIVE && (mine & kLossy))))
       a.out_vals[base + a.heads[u] - 1] = __longlong_as_double((long long)Op::finalize(last_of[u], L));
   }
-  if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.inexact, 1u);
+  if constexpr (Op::TENTATIVE) {
+    const bool again = __any_sync(0xffffffffu, bad);
+    if (again) {
+      if (lane == 0) {
+        atomicOr(a.need + u, kInvolved | kReclose);
+        *static_cast<volatile uint32_t*>(a.inexact) = 1u;
+      }
+      if (lane <= stop && (int32_t)(u - 1 - lane) >= 0) atomicOr(a.need + (u - 1 - lane), kInvolved);
+    }
+    if (walk) {
+      if (open && lane == 0) s_again = again;
+      __syncthreads();
+      const int32_t from = s_pos;
+      if (s_again)
+        for (int32_t v = from + (int32_t)t; v < (int32_t)(blockIdx.x * 8); v += 256) atomicOr(a.need + v, kInvolved);
+    }
+  }
 }
 
 // ------------------------------------------------------------------ scalar reductions
@@ -860,6 +916,7 @@ struct F64Layout {
   size_t clear;
   uint32_t* heads;
   uint32_t* base;
+  uint32_t* need;
   uint8_t* first;
   uint8_t* last;
   size_t total;
@@ -883,6 +940,7 @@ F64Layout f64_layout(void* ws, uint64_t n) {
   l.clear = 4 * sizeof(uint32_t);
   l.heads = c.take<uint32_t>(units + 1);
   l.base = c.take<uint32_t>(units + 1);
+  l.need = c.take<uint32_t>(units + 1);
   l.first = c.take<uint8_t>((units + 1) * partial);
   l.last = c.take<uint8_t>((units + 1) * partial);
   l.total = align_up(c.used + 256, 256);
@@ -909,6 +967,7 @@ rfx_status f64_dispatch_op(F64Args a, uint32_t op, void* ws, cudaStream_t s) {
   a.done = l.done;
   a.heads = l.heads;
   a.base = l.base;
+  a.need = l.need;
   a.first = l.first;
   a.last = l.last;
   a.inexact = l.inexact_pair;
@@ -919,12 +978,12 @@ rfx_status f64_dispatch_op(F64Args a, uint32_t op, void* ws, cudaStream_t s) {
   if (op == RFX_F64_MIN) return f64_run_units<KB, MinOp>(a, units, s);
   rfx_status st = f64_run_units<KB, PairOp>(a, units, s);
   if (st != RFX_OK) return st;
-  // each further pass runs on the device only if the one before lost bits
+  // each further pass runs on the device only if the one before lost bits, over the marked units
   a.gate = l.inexact_pair;
   a.inexact = l.inexact_narrow;
   a.emax = l.emax;
-  const int ge = persistent_grid((const void*)f64_emax, 256, 0, (a.n + 2047) / 2048);
-  RFX_CUDA_TRY(launch_chained(f64_emax, ge, 256, 0, s, a));
+  const int ge = persistent_grid((const void*)f64_emax, 256, 0, (units + 7) / 8);
+  RFX_CUDA_TRY(launch_chained(f64_emax, ge, 256, 0, s, a, units));
   st = f64_run_units<KB, SumOp<kNarrowLimbs>>(a, units, s);
   if (st != RFX_OK) return st;
   a.gate = l.inexact_narrow;

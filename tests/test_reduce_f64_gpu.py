@@ -373,3 +373,27 @@ def test_smaller_inputs_in_the_workspace_of_more(cuda):
         k = int(g.item())
         ek, es = O.reduce_f64_exact(keys[:n], vals[:n])
         assert k == es.shape[0] and np.array_equal(to_np(ok[:k]), ek) and _same_bits(to_np(ov[:k]), es), n
+
+
+@pytest.mark.parametrize("n,every", [(256 * 300, 60), (256 * 300, 1500), (256 * 700 + 13, 20_000), (256 * 700 + 13, 200_000),
+                                     (4737 * 256 * 3 + 100, 100_000)])
+@pytest.mark.parametrize("far", [1e-15, 1e-40, 1e300])
+@pytest.mark.parametrize("runs", ["short", "units", "long", "mixed"])
+def test_sum_with_some_units_done_over(cuda, n, every, far, runs):
+    """Amounts with a few values that the pair of doubles cannot hold beside them: the integer
+    passes do those values' units over and the units of the runs through them, and every sum, of
+    runs inside a unit, over a few units and over very many, beside others and through them, is exact."""
+    rng = np.random.default_rng(n + every + len(runs))
+    vals = gen_values("prices", n, every)
+    at = rng.integers(0, n, max(1, n // every))
+    vals[at] = far * rng.choice([1.0, -1.0], at.shape[0])
+    mean = {"short": 5, "units": 700, "long": 40_000, "mixed": 0}[runs]
+    if mean:
+        keys = np.sort(rng.integers(0, max(1, n // mean), n)).astype(np.uint32)
+    else:
+        lens = np.exp(rng.uniform(0, np.log(50_000), n // 1000 + 50)).astype(np.int64) + 1
+        keys = np.repeat(np.arange(lens.shape[0], dtype=np.uint32), lens)[:n]
+        keys = np.concatenate([keys, np.full(n - keys.shape[0], 1 << 20, np.uint32)])
+    ok, ov, g = R.reduce_f64(_dev(keys, cuda), _dev(vals, cuda), R.F64_SUM)
+    ek, es = O.reduce_f64_exact(keys, vals)
+    assert g == es.shape[0] and np.array_equal(to_np(ok), ek) and _same_bits(to_np(ov), es)
